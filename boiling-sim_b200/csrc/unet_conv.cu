@@ -1,43 +1,42 @@
 // unet_conv.cu -- the 3x3x3 convolutions of the warm-start network's training
 // pass on the unpadded layout act[v][c], v = (i ny + j) nz + k, channels
 // innermost (BF16), weights w[tap][co][ci] (tap = (di+1) 9 + (dj+1) 3 + (dk+1)):
-// the forward pass (and the data gradient, the same kernel on flipped
-// weights) on tcgen05 tensor cores, the weight and bias gradients on mma.sync.
+// forward (and data gradient, the same kernel on flipped weights), weight and
+// bias gradient.
 //
-// Forward.  A tile is 8 k x 16 j voxels of one i plane: the 128 rows (TMEM
-// lanes) of D.  Its input window, 10 k x 18 j rows of one plane, is staged
-// once per plane as [channel group of 8][j][k][16 bytes] -- exactly the
-// K-major no-swizzle core matrix (8 rows of 16 bytes), so the operand of tap
-// (dj, dk) is the same staged plane read through a descriptor whose start is
-// moved by ((dj+1) 10 + (dk+1)) 16 bytes, with 8-row groups (one j line) 160
-// bytes apart and the two 8-channel halves of a K step 2880 bytes apart.  A CTA
-// marches along i with the planes i-1, i, i+1 in a ring, so a plane is read
-// from L2 once per tile (1.4x its voxels) and feeds all 27 taps; gathering the
-// rows per tap instead read every voxel 27 times and left the tensor cores
-// waiting (143 us against 15 us here for 32 -> 32 channels at 64x64x48 on a
-// B200; the bound is shared-memory operand reads, 32 cycles per M = 128,
-// K = 16 MMA at these small N).  Rows outside the grid are zero-filled by the
-// copy.  Weights stay in shared memory: at most 64 input channels x NT output
-// channels with 64 NT <= 2048; more input channels run in passes that
-// accumulate in tensor memory.
+// All three are mma.sync m16n8k16 (BF16 operands, FP32 accumulators).  The
+// forward pass keeps one accumulation order per output -- taps ascending,
+// 16-channel chunks ascending inside a tap -- because the ReLU gradient takes
+// its mask from the sign of the rounded output: another order flips an output
+// near zero once in a few million, and with it a term of the gradients.
+// tcgen05 kernels of the same tiling gave the same times at these channel
+// counts (32 -> 32 at 64x64x48: 31 us; an M = 128 instruction costs the same at
+// N = 32 as at N = 96) in another order.
+//
+// Forward.  A tile is 8 k x 16 j voxels; a CTA marches along i with the tile's
+// input window (10 x 18 rows of all input channels) of each plane staged once by
+// cp.async, zero-filled outside the grid.  A plane adds to three output planes
+// (through di = +1, 0, -1), whose accumulators a warp keeps in registers, so an
+// operand row read from shared memory feeds three taps, and a plane is read
+// from L2 1.4 times; gathering the rows per tap read every voxel 27 times.
+// Weights of the CTA's output channels stay in shared memory.
 //
 // Weight gradient.  dw[tap][co][ci] = sum_v g[v][co] in[v + d][ci]: the
-// contraction runs over voxels and M x N is only 16 or 32 channels a side, so
-// mma.sync m16n8k16 fits it without padding (a 64 x 64 tile did 4-16 times the
-// work).  A CTA takes one di and a block of MC x NC channels; its nine warps
-// take the nine (dj, dk) taps from the same staged 128-voxel g tile and
-// 10 x 18 row input window: 358 us -> 22 us for the same layer.  Chains of MMA
-// accumulation are cut every 2048 voxels into a second set of FP32 registers.
-// The bias gradient is summed from the staged g tiles of di = 0.  Partial sums
-// per split are added in a fixed order (deterministic).
+// contraction runs over voxels, and M x N is a block of 16 or 32 channels a
+// side (a fixed 64 x 64 tile did 4 to 16 times the work of these layers).  The
+// nine warps of a CTA take the nine (dj, dk) taps; it marches along i with input
+// and gradient planes in rings, all three di from the same staged planes.
+// Chains of MMA accumulation are cut every 2048 voxels.  The bias gradient is
+// summed from the staged gradient planes.  Partial sums per split are added
+// in a fixed order (deterministic).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bsp_common.cuh"
-#include "tc5.cuh"
 
 namespace bsp {
 namespace uconv {
@@ -46,15 +45,11 @@ constexpr int TK = 8, TJ = 16;                 // voxels of a tile: 8 k x 16 j
 constexpr int WK = TK + 2, WJ = TJ + 2;        // its input window
 constexpr int WROWS = WK * WJ;                 // 180 rows
 constexpr int HALF = WROWS * 16;               // bytes of one 8-channel group of a plane
-constexpr int NPROD = 4;                       // producer warps
-constexpr int FWD_THREADS = (4 + 1 + NPROD) * 32;
-constexpr int MAXSLOT = 6, MAXACC = 8;
-constexpr int CP_MAX = 64;                     // input channels per pass
-constexpr int W_BYTES_MAX = 27 * 2048 * 2;     // weights of a pass: channels x NT <= 2048
 constexpr int SMEM_MAX = 232448;
 
-__device__ int g_conv_err;  // BSP_ERR_TIMEOUT once a bounded wait gave up
-
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool valid) {
   // src-size 0 zero-fills the 16 destination bytes
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
@@ -66,255 +61,13 @@ template <int N>
 __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-struct FwdArgs {
-  __nv_bfloat16 *out;
-  const __nv_bfloat16 *in, *w;
-  const float *bias;
-  int nx, ny, nz, cin, cout, relu;
-  int nt, nct;      // output channels per CTA, channel tiles
-  int jt, kt;       // tiles per plane
-  int len, npass;   // planes per CTA, input-channel passes
-  int cp;           // input channels of a full pass
-  int nslot, nacc;  // plane ring, accumulators
-  int wbytes, slot_bytes;
-  int vec;          // out rows are 16-byte aligned
-};
-
-struct FwdCtl {
-  uint64_t full[MAXSLOT], empty[MAXSLOT], acc_full[MAXACC], acc_empty[MAXACC], wfree, drain;
-  uint32_t tmem_base;
-  int abort;
-};
-
-__device__ __forceinline__ bool wait_ok(uint64_t *bar, uint32_t parity, FwdCtl *c) {
-  if (mbar_wait(bar, parity)) return true;
-  *(volatile int *)&c->abort = 1;
-  atomicExch(&g_conv_err, BSP_ERR_TIMEOUT);
-  return false;
+__device__ __forceinline__ void ldsm_x4(uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3,
+                                        uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr)
+               : "memory");
 }
-
-// Warps 0-3: epilogue (TMEM lane quarter = warp), warp 4: TMEM allocation and
-// MMA issue (one thread), warps 5-8: cp.async producers.
-// Plane fills are numbered f = pass (len + 2) + pl, pl = 0 .. len + 1 for plane
-// i0 - 1 + pl; fill f goes to slot f mod nslot.  Output o of a pass reads fills
-// o, o + 1, o + 2 of it; fill o is free after output o (the last two after the
-// last output).  A producer warp arrives for fill f only after its copies of
-// f + la are issued, la = nslot - 3 (at most 2): waiting for the slot of f
-// needs output f - nslot, i.e. fills up to f - nslot + 2 <= f - la - 1, which
-// have been arrived for.  The pass's weights are copied before its first
-// plane, so a full first plane implies them.
-__global__ void __launch_bounds__(FWD_THREADS, 2) conv_fwd_kernel(const FwdArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char *wsm = smem;
-  unsigned char *slots = smem + a.wbytes;
-  FwdCtl *c = reinterpret_cast<FwdCtl *>(slots + (size_t)a.nslot * a.slot_bytes);
-  int t = blockIdx.x;
-  const int ct = t % a.nct;
-  t /= a.nct;
-  const int k0 = (t % a.kt) * TK;
-  t /= a.kt;
-  const int j0 = (t % a.jt) * TJ;
-  const int i0 = (t / a.jt) * a.len;
-  const int len = min(a.len, a.nx - i0);
-  const int co0 = ct * a.nt;
-  const int nt = a.nt, npass = a.npass;
-  uint32_t tcols = 32;
-  while (tcols < (uint32_t)(a.nacc * nt)) tcols <<= 1;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < a.nslot; ++s) {
-      mbar_init(&c->full[s], NPROD);
-      mbar_init(&c->empty[s], 1);
-    }
-    for (int b = 0; b < a.nacc; ++b) {
-      mbar_init(&c->acc_full[b], 1);
-      mbar_init(&c->acc_empty[b], 4);
-    }
-    mbar_init(&c->wfree, 1);
-    mbar_init(&c->drain, 1);
-    c->abort = 0;
-    utc::fence_barrier_init();
-  }
-  if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&c->tmem_base)),
-                 "r"(tcols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  utc::fence_async_shared();
-  utc::tc_fence_before();
-  __syncthreads();
-  utc::tc_fence_after();
-  const uint32_t tbase = c->tmem_base;
-
-  if (warp >= 5) {
-    // ---------------- producers ----------------
-    const int pt = threadIdx.x - 160;  // 0 .. 127
-    const uint32_t wsm_u = smem_u32(wsm), slots_u = smem_u32(slots);
-    const int la = a.nslot >= 5 ? 2 : 1;
-    const int64_t plane = (int64_t)a.ny * a.nz;
-    int f = 0, arrived = 0;
-    bool ok = true;
-    auto arrive_next = [&]() {
-      utc::fence_async_shared();
-      __syncwarp();
-      if (lane == 0) utc::mbar_arrive(&c->full[arrived % a.nslot]);
-      ++arrived;
-    };
-    for (int ps = 0; ps < npass && ok; ++ps) {
-      const int c0 = ps * a.cp, cp = min(a.cp, a.cin - c0), cg = cp >> 3;
-      if (ps > 0) {
-        // the weight buffer is read by the MMAs of the pass before
-        cp_wait<0>();
-        while (arrived < f) arrive_next();
-        ok = __all_sync(0xffffffffu, wait_ok(&c->wfree, (uint32_t)((ps - 1) & 1), c));
-        if (!ok) break;
-      }
-      // weights: [tap][channel group of 8][n][16 bytes]
-      for (int q = pt; q < 27 * cg * nt; q += NPROD * 32) {
-        const int g8 = q % cg, r = q / cg;
-        const int n = r % nt, tap = r / nt;
-        cp16(wsm_u + (uint32_t)(((tap * cg + g8) * nt + n) * 16),
-             a.w + ((int64_t)tap * a.cout + co0 + n) * a.cin + c0 + g8 * 8, true);
-      }
-      for (int pl = 0; pl < len + 2; ++pl, ++f) {
-        const int s = f % a.nslot;
-        ok = __all_sync(0xffffffffu,
-                        wait_ok(&c->empty[s], (uint32_t)(((f / a.nslot) & 1) ^ 1), c));
-        if (!ok) break;
-        const int i = i0 - 1 + pl;
-        const bool iok = i >= 0 && i < a.nx;
-        const uint32_t dst = slots_u + (uint32_t)(s * a.slot_bytes);
-        for (int q = pt; q < WROWS * cg; q += NPROD * 32) {
-          const int row = q / cg, g8 = q - row * cg;
-          const int jj = row / WK, kk = row - jj * WK;
-          const int j = j0 - 1 + jj, k = k0 - 1 + kk;
-          const bool v = iok && j >= 0 && j < a.ny && k >= 0 && k < a.nz;
-          const __nv_bfloat16 *src =
-              v ? a.in + (i * plane + (int64_t)j * a.nz + k) * a.cin + c0 + g8 * 8 : a.in;
-          cp16(dst + (uint32_t)(g8 * HALF + row * 16), src, v);
-        }
-        cp_commit();
-        if (f - arrived >= la) {
-          if (la == 2)
-            cp_wait<2>();
-          else
-            cp_wait<1>();
-          arrive_next();
-        }
-      }
-    }
-    cp_wait<0>();
-    if (ok)
-      while (arrived < f) arrive_next();
-  } else if (warp == 4) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = utc::idesc_bf16(nt, 128);
-      const uint32_t wsm_u = smem_u32(wsm), slots_u = smem_u32(slots);
-      bool ok = true;
-      for (int ps = 0; ps < npass && ok; ++ps) {
-        const int cp = min(a.cp, a.cin - ps * a.cp), cg = cp >> 3;
-        const int f0 = ps * (len + 2);
-        const uint64_t bstep = (uint64_t)(cg * nt);  // 16-byte units per tap
-        for (int o = 0; o < len && ok; ++o) {
-          const int b = o % a.nacc;
-          if (npass == 1) ok = wait_ok(&c->acc_empty[b], (uint32_t)(((o / a.nacc) & 1) ^ 1), c);
-          for (int x = o == 0 ? 0 : 2; x < 3 && ok; ++x) {
-            const int f = f0 + o + x;
-            ok = wait_ok(&c->full[f % a.nslot], (uint32_t)((f / a.nslot) & 1), c);
-          }
-          if (!ok) break;
-          utc::tc_fence_after();
-          const uint32_t dt = tbase + (uint32_t)(b * nt);
-          uint32_t acc = ps > 0 ? 1u : 0u;
-          for (int di = 0; di < 3; ++di) {
-            const uint32_t sl = slots_u + (uint32_t)(((f0 + o + di) % a.nslot) * a.slot_bytes);
-            for (int kc = 0; kc < cg / 2; ++kc) {
-              const uint64_t ad = utc::sdesc(sl + (uint32_t)(kc * 2 * HALF), HALF, WK * 16);
-              const uint64_t bd = utc::sdesc(
-                  wsm_u + (uint32_t)(((di * 9 * cg) + kc * 2) * nt * 16), nt * 16, 128);
-#pragma unroll
-              for (int s = 0; s < 9; ++s) {
-                utc::tc_mma(dt, ad + (uint64_t)((s / 3) * WK + s % 3), bd + (uint64_t)s * bstep,
-                            idesc, acc);
-                acc = 1u;
-              }
-            }
-          }
-          utc::tc_commit(&c->empty[(f0 + o) % a.nslot]);
-          if (o == len - 1) {
-            utc::tc_commit(&c->empty[(f0 + len) % a.nslot]);
-            utc::tc_commit(&c->empty[(f0 + len + 1) % a.nslot]);
-          }
-          if (ps == npass - 1) utc::tc_commit(&c->acc_full[b]);
-        }
-        if (ok && ps + 1 < npass) utc::tc_commit(&c->wfree);
-      }
-      // drain: every MMA issued has completed before TMEM is freed
-      utc::tc_commit(&c->drain);
-      mbar_wait(&c->drain, 0);
-    }
-  } else {
-    // ---------------- epilogue ----------------
-    const int row = warp * 32 + lane;
-    const int j = j0 + (row >> 3), k = k0 + (row & 7);
-    const bool valid = j < a.ny && k < a.nz;
-    for (int o = 0; o < len; ++o) {
-      const int b = o % a.nacc;
-      if (!__all_sync(0xffffffffu,
-                      wait_ok(&c->acc_full[b], (uint32_t)((o / a.nacc) & 1), c)))
-        break;
-      utc::tc_fence_after();
-      const uint32_t trow = tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * nt);
-      const int64_t v = ((int64_t)(i0 + o) * a.ny + j) * a.nz + k;
-      for (int cb = 0; cb < nt; cb += 16) {
-        float x[16];
-        utc::tmem_ld1x16(trow + (uint32_t)cb, x);
-        if (!valid) continue;
-        if (a.bias) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) x[e] += __ldg(a.bias + co0 + cb + e);
-        }
-        if (a.relu) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) x[e] = fmaxf(x[e], 0.0f);
-        }
-        uint32_t w[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = utc::pack_bf16x2(x[2 * e], x[2 * e + 1]);
-        __nv_bfloat16 *dst = a.out + v * a.cout + co0 + cb;
-        if (a.vec) {
-          reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) reinterpret_cast<uint32_t *>(dst)[e] = w[e];
-        }
-      }
-      utc::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) utc::mbar_arrive(&c->acc_empty[b]);
-    }
-  }
-  utc::tc_fence_before();
-  __syncthreads();
-  utc::tc_fence_after();
-  if (warp == 4)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase),
-                 "r"(tcols)
-                 : "memory");
-}
-
-// ---- weight and bias gradient -------------------------------------------------------------
-constexpr int WG_VCH = 2048;      // voxels per partial-sum slot of the workspace
-constexpr int WG_THREADS = 288;   // nine warps, one (dj, dk) tap each
-constexpr int WG_FLUSH = 16;      // tiles (2048 voxels) per MMA accumulation chain
-constexpr int WG_STAGES = 3;
-
 __device__ __forceinline__ void ldsm_x4_t(uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3,
                                           uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -331,16 +84,304 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+struct FwdArgs {
+  __nv_bfloat16 *out;
+  const __nv_bfloat16 *in, *w;
+  const float *bias;
+  int nx, ny, nz, cout, relu;
+  int nct;     // output-channel tiles
+  int jt, kt;  // tiles per plane
+  int len;     // output planes per CTA
+};
+
+// CIN input channels, NT output channels per CTA, MT 16-row blocks per warp
+// (8 / MT warps of 16 MT voxels each), NS plane slots.
+template <int CIN, int NT, int MT, int NS>
+struct FwdShape {
+  static constexpr int WARPS = 8 / MT, THREADS = WARPS * 32;
+  static constexpr int PITCH = CIN * 2 + 16;  // bytes of a staged row
+  static constexpr int W_BYTES = 27 * NT * PITCH, SLOT = WROWS * PITCH;
+  static constexpr int SMEM = W_BYTES + NS * SLOT;
+};
+
+template <int CIN, int NT, int MT, int NS>
+__global__ void __launch_bounds__(FwdShape<CIN, NT, MT, NS>::THREADS)
+    conv_fwd_kernel(const FwdArgs a) {
+  using S = FwdShape<CIN, NT, MT, NS>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int PITCH = S::PITCH, CG = CIN / 8, NK = CIN / 16, NG = NT / 16;
+  constexpr int XQ = (WROWS * CG + S::THREADS - 1) / S::THREADS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int t = blockIdx.x;
+  const int co0 = (t % a.nct) * NT;
+  t /= a.nct;
+  const int k0 = (t % a.kt) * TK;
+  t /= a.kt;
+  const int j0 = (t % a.jt) * TJ;
+  const int i0 = (t / a.jt) * a.len;
+  const int len = min(a.len, a.nx - i0);
+  const uint32_t wsm = smem_u32(smem), slots = wsm + S::W_BYTES;
+  // weights: [tap][n] rows of CIN channels
+  for (int q = tid; q < 27 * NT * CG; q += S::THREADS) {
+    const int row = q / CG, g8 = q % CG;
+    const int tap = row / NT, n = row % NT;
+    cp16(wsm + (uint32_t)(row * PITCH + g8 * 16),
+         a.w + ((int64_t)tap * a.cout + co0 + n) * CIN + g8 * 8, true);
+  }
+  // this thread's pieces of an input window
+  int xoff[XQ];
+  uint32_t xok = 0;
+#pragma unroll
+  for (int q = 0; q < XQ; ++q) {
+    const int p = tid + q * S::THREADS, row = p / CG;
+    const int j = j0 - 1 + row / WK, k = k0 - 1 + row % WK;
+    xoff[q] = (j * a.nz + k) * CIN + (p % CG) * 8;
+    if (row < WROWS && (unsigned)j < (unsigned)a.ny && (unsigned)k < (unsigned)a.nz)
+      xok |= 1u << q;
+  }
+  static_assert(XQ <= 32 && S::THREADS % CG == 0, "piece layout");
+  const uint32_t xdst = (uint32_t)((tid / CG) * PITCH + (tid % CG) * 16);
+  const int64_t plane = (int64_t)a.ny * a.nz * CIN;
+  auto stage = [&](int pl, int s) {
+    const int i = i0 - 1 + pl;
+    const bool iok = (unsigned)i < (unsigned)a.nx;
+    const __nv_bfloat16 *src = a.in + (iok ? i * plane : 0);
+#pragma unroll
+    for (int q = 0; q < XQ; ++q) {
+      const bool v = iok && (xok >> q & 1);
+      if (XQ * S::THREADS == WROWS * CG || tid + q * S::THREADS < WROWS * CG)
+        cp16(slots + (uint32_t)(s * S::SLOT) + xdst +
+                 (uint32_t)(q * (S::THREADS / CG) * PITCH),
+             v ? src + xoff[q] : a.in, v);
+    }
+  };
+  // operand addresses of this lane
+  const int r = warp * 16 * MT + (lane & 15);  // voxel row of the first block
+  const uint32_t xa = (uint32_t)(((r >> 3) * WK + (r & 7)) * PITCH + (lane >> 4) * 16);
+  const uint32_t wa = wsm + (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * PITCH +
+                                       ((lane >> 3) & 1) * 16);
+  // accumulators of outputs pl - 2, pl - 1, pl (through di = +1, 0, -1)
+  float acc[3][MT][2 * NG][4];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < 2 * NG; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[d][m][n][q] = 0.0f;
+#pragma unroll
+  for (int s = 0; s < NS - 1; ++s) {
+    if (s < len + 2) stage(s, s);
+    cp_commit();
+  }
+  int slot = 0;
+  for (int pl = 0; pl < len + 2; ++pl) {
+    cp_wait<NS - 2>();
+    __syncthreads();  // plane pl staged by every thread; plane pl - 1 no longer read
+    if (pl + NS - 1 < len + 2) stage(pl + NS - 1, slot == 0 ? NS - 1 : slot - 1);
+    cp_commit();
+    const uint32_t xs = slots + (uint32_t)(slot * S::SLOT) + xa;
+    const bool use[3] = {pl >= 2, pl >= 1 && pl <= len, pl < len};
+#pragma unroll 1
+    for (int dj = 0; dj < 3; ++dj) {
+#pragma unroll
+      for (int dk = 0; dk < 3; ++dk) {
+#pragma unroll
+        for (int kc = 0; kc < NK; ++kc) {
+          uint32_t A[MT][4];
+#pragma unroll
+          for (int m = 0; m < MT; ++m)
+            ldsm_x4(A[m][0], A[m][1], A[m][2], A[m][3],
+                    xs + (uint32_t)((dj + 2 * m) * WK * PITCH + dk * PITCH + kc * 32));
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            if (!use[d]) continue;
+            const uint32_t wt = wa + (uint32_t)((((2 - d) * 9 + dk) * NT) * PITCH + kc * 32) +
+                                (uint32_t)(dj * 3 * NT * PITCH);
+#pragma unroll
+            for (int n = 0; n < NG; ++n) {
+              uint32_t b0, b1, b2, b3;
+              ldsm_x4(b0, b1, b2, b3, wt + (uint32_t)(n * 16 * PITCH));
+#pragma unroll
+              for (int m = 0; m < MT; ++m) {
+                mma_bf16(acc[d][m][2 * n], A[m], b0, b1);
+                mma_bf16(acc[d][m][2 * n + 1], A[m], b2, b3);
+              }
+            }
+          }
+        }
+      }
+    }
+    if (pl >= 2) {  // output pl - 2 is complete
+      const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int row = warp * 16 * MT + m * 16 + g + h * 8;
+          const int j = j0 + (row >> 3), k = k0 + (row & 7);
+          if (j >= a.ny || k >= a.nz) continue;
+          const int64_t v = ((int64_t)(i0 + pl - 2) * a.ny + j) * a.nz + k;
+#pragma unroll
+          for (int n = 0; n < 2 * NG; ++n) {
+            const int co = co0 + n * 8 + t4 * 2;
+            float x0 = acc[0][m][n][2 * h], x1 = acc[0][m][n][2 * h + 1];
+            if (a.bias) {
+              x0 += a.bias[co];
+              x1 += a.bias[co + 1];
+            }
+            if (a.relu) {
+              x0 = fmaxf(x0, 0.0f);
+              x1 = fmaxf(x1, 0.0f);
+            }
+            *reinterpret_cast<__nv_bfloat162 *>(a.out + v * a.cout + co) =
+                __floats2bfloat162_rn(x0, x1);
+          }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < 2 * NG; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc[0][m][n][q] = acc[1][m][n][q];
+          acc[1][m][n][q] = acc[2][m][n][q];
+          acc[2][m][n][q] = 0.0f;
+        }
+    slot = slot + 1 == NS ? 0 : slot + 1;
+  }
+}
+
+// Any channel counts (multiples of 16): one tap and 16 channels per step,
+// rows gathered per tap.  Serves the input-channel counts that have no staged
+// kernel above (no layer of the network).
+constexpr int GM = 128, GROW = 48;  // voxels per CTA; bytes of a staged row
+template <int NT>
+__global__ void __launch_bounds__(GM) conv_any_kernel(FwdArgs a, int cin) {
+  __shared__ __align__(128) unsigned char sA[2][GM * GROW];
+  __shared__ __align__(128) unsigned char sB[2][NT * GROW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t nvox = (int64_t)a.nx * a.ny * a.nz, v0 = (int64_t)blockIdx.x * GM;
+  const int co0 = blockIdx.y * NT;
+  const int64_t va = v0 + tid;
+  const bool vin = va < nvox;
+  const int ka = vin ? (int)(va % a.nz) : 0;
+  const int ja = vin ? (int)(va / a.nz % a.ny) : 0, ia = vin ? (int)(va / a.nz / a.ny) : 0;
+  const int nk = cin >> 4, steps = 27 * nk;
+  auto stage = [&](int s, int buf) {
+    const int tap = s / nk, c0 = (s - tap * nk) << 4;
+    const int ii = ia + tap / 9 - 1, jj = ja + tap / 3 % 3 - 1, kk = ka + tap % 3 - 1;
+    const bool ok = vin && (unsigned)ii < (unsigned)a.nx && (unsigned)jj < (unsigned)a.ny &&
+                    (unsigned)kk < (unsigned)a.nz;
+    const __nv_bfloat16 *src = ok ? a.in + (((int64_t)ii * a.ny + jj) * a.nz + kk) * cin + c0 : a.in;
+    const uint32_t dst = smem_u32(sA[buf] + tid * GROW);
+    cp16(dst, src, ok);
+    cp16(dst + 16, ok ? src + 8 : src, ok);
+    for (int r = tid; r < NT * 2; r += GM)
+      cp16(smem_u32(sB[buf] + (r >> 1) * GROW + (r & 1) * 16),
+           a.w + ((int64_t)tap * a.cout + co0 + (r >> 1)) * cin + c0 + (r & 1) * 8, true);
+    cp_commit();
+  };
+  float acc[2][NT / 8][4] = {};
+  stage(0, 0);
+  for (int s = 0; s < steps; ++s) {
+    const int buf = s & 1;
+    if (s + 1 < steps) {
+      stage(s + 1, buf ^ 1);
+      cp_wait<1>();
+    } else {
+      cp_wait<0>();
+    }
+    __syncthreads();
+    uint32_t A[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      ldsm_x4(A[m][0], A[m][1], A[m][2], A[m][3],
+              smem_u32(sA[buf] + (warp * 32 + m * 16 + (lane & 15)) * GROW + (lane >> 4) * 16));
+#pragma unroll
+    for (int n = 0; n < NT / 16; ++n) {
+      uint32_t b0, b1, b2, b3;
+      ldsm_x4(b0, b1, b2, b3,
+              smem_u32(sB[buf] + (n * 16 + (lane >> 4) * 8 + (lane & 7)) * GROW +
+                       ((lane >> 3) & 1) * 16));
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        mma_bf16(acc[m][2 * n], A[m], b0, b1);
+        mma_bf16(acc[m][2 * n + 1], A[m], b2, b3);
+      }
+    }
+    __syncthreads();
+  }
+  const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t v = v0 + warp * 32 + m * 16 + g + h * 8;
+      if (v >= nvox) continue;
+#pragma unroll
+      for (int n = 0; n < NT / 8; ++n) {
+        const int co = co0 + n * 8 + t4 * 2;
+        float x0 = acc[m][n][2 * h], x1 = acc[m][n][2 * h + 1];
+        if (a.bias) {
+          x0 += a.bias[co];
+          x1 += a.bias[co + 1];
+        }
+        if (a.relu) {
+          x0 = fmaxf(x0, 0.0f);
+          x1 = fmaxf(x1, 0.0f);
+        }
+        *reinterpret_cast<__nv_bfloat162 *>(a.out + v * a.cout + co) =
+            __floats2bfloat162_rn(x0, x1);
+      }
+    }
+}
+
+template <int CIN, int NT, int MT, int NS>
+cudaError_t launch_fwd(FwdArgs a, cudaStream_t s) {
+  using S = FwdShape<CIN, NT, MT, NS>;
+  static_assert(S::SMEM <= SMEM_MAX, "shared memory");
+  auto kern = conv_fwd_kernel<CIN, NT, MT, NS>;
+  if (!smem_opt_in((const void *)kern, S::SMEM)) return cudaErrorNotSupported;
+  a.nct = a.cout / NT;
+  a.jt = (a.ny + TJ - 1) / TJ;
+  a.kt = (a.nz + TK - 1) / TK;
+  // Planes per CTA: waves x (planes + the two halo planes, which cost a third
+  // of the MMAs each, + about two planes' time for loading the weights) least.
+  const int occ = std::max(1, std::min(SMEM_MAX / (S::SMEM + 1024), MT == 2 ? 3 : 1));
+  const int64_t cols = (int64_t)a.jt * a.kt * a.nct, slots = 148 * occ;
+  int64_t best = INT64_MAX;
+  for (int l = 1; l <= a.nx; ++l) {
+    const int64_t items = cols * ((a.nx + l - 1) / l);
+    const int64_t cost = ((items + slots - 1) / slots) * (l + 3);
+    if (cost <= best) {
+      best = cost;
+      a.len = l;
+    }
+  }
+  const int64_t items = cols * ((a.nx + a.len - 1) / a.len);
+  if (items > 0x7fffffff) return cudaErrorInvalidValue;
+  kern<<<(unsigned)items, S::THREADS, S::SMEM, s>>>(a);
+  return cudaGetLastError();
+}
+
+// ---- weight and bias gradient -------------------------------------------------------------
+constexpr int WG_VCH = 2048;      // voxels per partial-sum slot of the workspace
+constexpr int WG_THREADS = 288;   // nine warps, one (dj, dk) tap each
+constexpr int WG_FLUSH = 16;      // tiles (2048 voxels) per MMA accumulation chain
+
 // Row pitches of C channels: C * 2 + 16 bytes put eight consecutive rows on
-// distinct banks for ldmatrix (48 and 80 bytes).
-template <int MC, int NC>
-constexpr int wg_stage_bytes() {
-  return TK * TJ * (MC * 2 + 16) + WROWS * (NC * 2 + 16);
-}
-template <int MC, int NC>
-constexpr int wg_smem_bytes() {
-  return WG_STAGES * wg_stage_bytes<MC, NC>() + 64;
-}
+// distinct banks for ldmatrix (48 and 80 bytes).  ND: the di a CTA computes,
+// all three (planes in a ring of 5 slots) or one.
+template <int MC, int NC, int ND>
+struct WgShape {
+  static constexpr int GP = MC * 2 + 16, XP = NC * 2 + 16;
+  static constexpr int GB = TK * TJ * GP, XB = WROWS * XP;
+  static constexpr int GS = 3, XS = 2 + ND;  // slots: two steps ahead
+  static constexpr int SMEM = GS * GB + XS * XB + 64;
+};
 
 struct WgArgs {
   float *dst;    // splits == 1: dw; else split s's [27][cout][cin] at s * 27 cout cin
@@ -348,134 +389,194 @@ struct WgArgs {
   const __nv_bfloat16 *g, *in;
   int nx, ny, nz, cin, cout;
   int jt, kt, nbi;  // tiles per plane, input-channel blocks
-  int64_t tiles;
+  int64_t tiles;    // (j, k) tiles x planes, plane index fastest
 };
 
-template <int MC, int NC>
-__global__ void __launch_bounds__(WG_THREADS, 2) conv_wgrad_kernel(const WgArgs a) {
+template <int MC, int NC, int ND>
+__global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(const WgArgs a) {
+  using S = WgShape<MC, NC, ND>;
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int GP = MC * 2 + 16, XP = NC * 2 + 16;  // row pitches
-  constexpr int GB = TK * TJ * GP, SB = wg_stage_bytes<MC, NC>();
-  constexpr int GC = MC / 8, XC = NC / 8;            // 16-byte pieces per row
+  constexpr int GP = S::GP, XP = S::XP, GS = S::GS, XS = S::XS;
+  constexpr int GC = MC / 8, XC = NC / 8;  // 16-byte pieces per row
+  constexpr int GQ = (TK * TJ * GC + WG_THREADS - 1) / WG_THREADS;  // pieces per thread
+  constexpr int XQ = (WROWS * XC + WG_THREADS - 1) / WG_THREADS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int di = (int)blockIdx.y % 3 - 1, blk = (int)blockIdx.y / 3;
+  // grid.y: channel block, and the di with ND = 1
+  const int blk = ND == 3 ? (int)blockIdx.y : (int)blockIdx.y / 3;
+  const int di0 = ND == 3 ? -1 : (int)blockIdx.y % 3 - 1;  // first di
   const int co0 = (blk / a.nbi) * MC, ci0 = (blk % a.nbi) * NC;
   const int dj = warp / 3, dk = warp % 3;  // + 1
-  const int64_t t0 = a.tiles * blockIdx.x / gridDim.x, t1 = a.tiles * (blockIdx.x + 1) / gridDim.x;
-  const uint32_t base = smem_u32(smem), zrow = base + WG_STAGES * SB;
-  if (tid < 4) *reinterpret_cast<uint4 *>(smem + WG_STAGES * SB + tid * 16) = make_uint4(0, 0, 0, 0);
-  auto coords = [&](int64_t t, int &i, int &j0, int &k0) {
-    k0 = (int)(t % a.kt) * TK;
-    t /= a.kt;
-    j0 = (int)(t % a.jt) * TJ;
-    i = (int)(t / a.jt);
-  };
-  auto stage = [&](int64_t t, int s) {
-    int i, j0, k0;
-    coords(t, i, j0, k0);
-    const uint32_t gs = base + s * SB, xs = gs + GB;
-    for (int q = tid; q < TK * TJ * GC; q += WG_THREADS) {
-      const int row = q / GC, p = q % GC;
-      const int j = j0 + row / TK, k = k0 + row % TK;
-      const bool v = j < a.ny && k < a.nz;
-      cp16(gs + row * GP + p * 16,
-           v ? a.g + (((int64_t)i * a.ny + j) * a.nz + k) * a.cout + co0 + p * 8 : a.g, v);
-    }
-    const int ii = i + di;
-    const bool iok = ii >= 0 && ii < a.nx;
-    for (int q = tid; q < WROWS * XC; q += WG_THREADS) {
-      const int row = q / XC, p = q % XC;
-      const int jj = row / WK, j = j0 - 1 + jj, k = k0 - 1 + row - jj * WK;
-      const bool v = iok && j >= 0 && j < a.ny && k >= 0 && k < a.nz;
-      cp16(xs + row * XP + p * 16,
-           v ? a.in + (((int64_t)ii * a.ny + j) * a.nz + k) * a.cin + ci0 + p * 8 : a.in, v);
-    }
-  };
-  float acc[MC / 16][NC / 8][4], sum[MC / 16][NC / 8][4];
+  int64_t t = a.tiles * blockIdx.x / gridDim.x;
+  const int64_t t1 = a.tiles * (blockIdx.x + 1) / gridDim.x;
+  const uint32_t gbase = smem_u32(smem), xbase = gbase + GS * S::GB, zrow = xbase + XS * S::XB;
+  if (tid < 4)
+    *reinterpret_cast<uint4 *>(smem + GS * S::GB + XS * S::XB + tid * 16) = make_uint4(0, 0, 0, 0);
+  static_assert(WG_THREADS % GC == 0 && WG_THREADS % XC == 0, "pieces of a thread share a column");
+  const uint32_t gdst = gbase + (uint32_t)((tid / GC) * GP + (tid % GC) * 16);
+  const uint32_t xdst = xbase + (uint32_t)((tid / XC) * XP + (tid % XC) * 16);
+  float acc[ND][MC / 16][NC / 8][4];
+  auto clear = [&]() {
 #pragma unroll
-  for (int m = 0; m < MC / 16; ++m)
-#pragma unroll
-    for (int n = 0; n < NC / 8; ++n)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[m][n][q] = sum[m][n][q] = 0.0f;
-  const bool bias = a.dbdst != nullptr && di == 0 && ci0 == 0;
-  constexpr int BG = WG_THREADS / MC;  // row groups of the bias sums
-  float bsum = 0.0f;
-  const int mat = lane >> 3, r = lane & 7;
-#pragma unroll
-  for (int s = 0; s < WG_STAGES - 1; ++s) {
-    if (t0 + s < t1) stage(t0 + s, s);
-    cp_commit();
-  }
-  int buf = 0, chain = 0;
-  for (int64_t t = t0; t < t1; ++t) {
-    cp_wait<WG_STAGES - 2>();
-    __syncthreads();  // tile t staged by every thread; tile t - 1 no longer read
-    if (t + WG_STAGES - 1 < t1) stage(t + WG_STAGES - 1, (buf + WG_STAGES - 1) % WG_STAGES);
-    cp_commit();
-    int i, j0, k0;
-    coords(t, i, j0, k0);
-    const uint32_t gs = base + buf * SB, xs = gs + GB;
-    const bool kok = k0 + r < a.nz;
-#pragma unroll
-    for (int ks = 0; ks < TJ / 2; ++ks) {
-      uint32_t A[MC / 16][4];
-#pragma unroll
-      for (int m = 0; m < MC / 16; ++m)
-        // A = g^T (co x v): rows v, columns co, read transposed
-        ldsm_x4_t(A[m][0], A[m][1], A[m][2], A[m][3],
-                  gs + (ks * 16 + (mat >> 1) * 8 + r) * GP + (m * 16 + (mat & 1) * 8) * 2);
-      const int jj = ks * 2 + (mat & 1);
-      // voxels past the grid's end read a zero row, so that their zero
-      // gradient meets no value of a neighbour
-      const bool v = kok && j0 + jj < a.ny;
-      const uint32_t xr = xs + ((jj + dj) * WK + r + dk) * XP;
-#pragma unroll
-      for (int n = 0; n < NC / 8; n += 2) {
-        uint32_t b0, b1, b2, b3;
-        const uint32_t off = (uint32_t)((n + (mat >> 1)) * 16);
-        ldsm_x4_t(b0, b1, b2, b3, (v ? xr : zrow) + off);
-#pragma unroll
-        for (int m = 0; m < MC / 16; ++m) {
-          mma_bf16(acc[m][n], A[m], b0, b1);
-          mma_bf16(acc[m][n + 1], A[m], b2, b3);
-        }
-      }
-    }
-    if (bias && tid < BG * MC) {
-      const __nv_bfloat16 *gp =
-          reinterpret_cast<const __nv_bfloat16 *>(smem + buf * SB) + tid % MC;
-      for (int row = tid / MC; row < TK * TJ; row += BG)
-        bsum += __bfloat162float(gp[row * (GP / 2)]);
-    }
-    if (++chain == WG_FLUSH) {
-      chain = 0;
+    for (int d = 0; d < ND; ++d)
 #pragma unroll
       for (int m = 0; m < MC / 16; ++m)
 #pragma unroll
         for (int n = 0; n < NC / 8; ++n)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            sum[m][n][q] += acc[m][n][q];
-            acc[m][n][q] = 0.0f;
+          for (int q = 0; q < 4; ++q) acc[d][m][n][q] = 0.0f;
+  };
+  // adds the accumulators to this split's sums (each element belongs to one
+  // thread of one CTA)
+  bool stored = false;
+  auto flush = [&]() {
+    const int g4 = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      float *dst = a.dst + ((int64_t)blockIdx.x * 27 + (di0 + d + 1) * 9 + warp) * a.cout * a.cin;
+#pragma unroll
+      for (int m = 0; m < MC / 16; ++m)
+#pragma unroll
+        for (int n = 0; n < NC / 8; ++n)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int co = co0 + m * 16 + g4 + h * 8, ci = ci0 + n * 8 + t4 * 2;
+            float *p = dst + (int64_t)co * a.cin + ci;
+            const float v0 = stored ? p[0] : 0.0f, v1 = stored ? p[1] : 0.0f;
+            p[0] = v0 + acc[d][m][n][2 * h];
+            p[1] = v1 + acc[d][m][n][2 * h + 1];
           }
     }
-    buf = buf + 1 == WG_STAGES ? 0 : buf + 1;
-  }
-  const int g4 = lane >> 2, t4 = lane & 3;
-  const int tap = (di + 1) * 9 + warp;
-  float *dst = a.dst + ((int64_t)blockIdx.x * 27 + tap) * a.cout * a.cin;
+    stored = true;
+    clear();
+  };
+  clear();
+  const bool bias = a.dbdst != nullptr && (ND == 3 || di0 == 0) && ci0 == 0;
+  constexpr int BG = WG_THREADS / MC;  // row groups of the bias sums
+  float bsum = 0.0f;
+  const int mat = lane >> 3, r = lane & 7;
+  const uint32_t ga = gbase + (uint32_t)(((mat >> 1) * 8 + r) * GP + (mat & 1) * 16);
+  const uint32_t xa =
+      xbase + (uint32_t)((((mat & 1) + dj) * WK + r + dk) * XP + (mat >> 1) * 16);
+  int chain = 0;
+  // runs of planes ia .. ib - 1 of one (j, k) tile
+  while (t < t1) {
+    const int col = (int)(t / a.nx), ia = (int)(t - (int64_t)col * a.nx);
+    const int ib = (int)(t1 - t < a.nx - ia ? ia + (t1 - t) : a.nx);
+    t += ib - ia;
+    const int k0 = col % a.kt * TK, j0 = col / a.kt * TJ;
+    // this thread's pieces of the tile's planes
+    int64_t goff[GQ], xoff[XQ];
+    uint32_t ok = 0;
 #pragma unroll
-  for (int m = 0; m < MC / 16; ++m)
+    for (int q = 0; q < GQ; ++q) {
+      const int row = (tid + q * WG_THREADS) / GC, j = j0 + row / TK, k = k0 + row % TK;
+      goff[q] = ((int64_t)j * a.nz + k) * a.cout + co0 + ((tid + q * WG_THREADS) % GC) * 8;
+      if (row < TK * TJ && j < a.ny && k < a.nz) ok |= 1u << q;
+    }
 #pragma unroll
-    for (int n = 0; n < NC / 8; ++n)
+    for (int q = 0; q < XQ; ++q) {
+      const int row = (tid + q * WG_THREADS) / XC, j = j0 - 1 + row / WK, k = k0 - 1 + row % WK;
+      xoff[q] = ((int64_t)j * a.nz + k) * a.cin + ci0 + ((tid + q * WG_THREADS) % XC) * 8;
+      if (row < WROWS && (unsigned)j < (unsigned)a.ny && (unsigned)k < (unsigned)a.nz)
+        ok |= 1u << (8 + q);
+    }
+    const int64_t gplane = (int64_t)a.ny * a.nz * a.cout, xplane = (int64_t)a.ny * a.nz * a.cin;
+    // step q stages input plane ia + di0 + q and gradient plane ia + q - (ND - 1),
+    // and computes that gradient plane on input planes of steps q - (ND - 1) .. q
+    const int nstep = ib - ia + ND - 1;
+    auto stage = [&](int q, int xs, int gs) {
+      const int i = ia + di0 + q;
+      const bool iok = (unsigned)i < (unsigned)a.nx;
+      const __nv_bfloat16 *x0 = a.in + (iok ? i * xplane : 0);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int co = co0 + m * 16 + g4 + h * 8, ci = ci0 + n * 8 + t4 * 2;
-        float *d = dst + (int64_t)co * a.cin + ci;
-        d[0] = sum[m][n][2 * h] + acc[m][n][2 * h];
-        d[1] = sum[m][n][2 * h + 1] + acc[m][n][2 * h + 1];
+      for (int p = 0; p < XQ; ++p) {
+        const bool v = iok && (ok >> (8 + p) & 1);
+        if (XQ * WG_THREADS == WROWS * XC || tid + p * WG_THREADS < WROWS * XC)
+          cp16(xdst + (uint32_t)(xs * S::XB + p * (WG_THREADS / XC) * XP), v ? x0 + xoff[p] : a.in,
+               v);
       }
+      if (q < ND - 1) return;
+      const __nv_bfloat16 *g0 = a.g + (ia + q - (ND - 1)) * gplane;
+#pragma unroll
+      for (int p = 0; p < GQ; ++p) {
+        const bool v = ok >> p & 1;
+        if (GQ * WG_THREADS == TK * TJ * GC || tid + p * WG_THREADS < TK * TJ * GC)
+          cp16(gdst + (uint32_t)(gs * S::GB + p * (WG_THREADS / GC) * GP), v ? g0 + goff[p] : a.g,
+               v);
+      }
+    };
+    const bool part = j0 + TJ > a.ny || k0 + TK > a.nz;
+    const bool kok = k0 + r < a.nz;
+    __syncthreads();  // the run before no longer reads its slots
+    stage(0, 0, 0);
+    cp_commit();
+    if (1 < nstep) stage(1, 1, 1);
+    cp_commit();
+    int xs = 0, gs = 0;
+    for (int q = 0; q < nstep; ++q) {
+      cp_wait<1>();
+      __syncthreads();  // step q staged by every thread; step q - 1 no longer reads
+      const int xn = xs + 2 >= XS ? xs + 2 - XS : xs + 2, gn = gs + 2 >= GS ? gs + 2 - GS : gs + 2;
+      if (q + 2 < nstep) stage(q + 2, xn, gn);
+      cp_commit();
+      if (q >= ND - 1) {
+        const uint32_t gb = ga + (uint32_t)(gs * S::GB);
+        uint32_t xb[ND];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          const int sl = xs - (ND - 1) + d;
+          xb[d] = xa + (uint32_t)((sl < 0 ? sl + XS : sl) * S::XB);
+        }
+        // Voxels past the grid's end read a zero input row, so that their
+        // zero gradient meets no value of a neighbour (only tiles that reach
+        // past it pay for the select).
+        auto plane_mma = [&](auto pt) {
+          constexpr bool PART = decltype(pt)::value;
+#pragma unroll
+          for (int ks = 0; ks < TJ / 2; ++ks) {
+            uint32_t A[MC / 16][4];
+#pragma unroll
+            for (int m = 0; m < MC / 16; ++m)
+              // A = g^T (co x v): rows v, columns co, read transposed
+              ldsm_x4_t(A[m][0], A[m][1], A[m][2], A[m][3],
+                        gb + (uint32_t)(ks * 16 * GP + m * 32));
+            const bool zr = PART && !(kok && j0 + ks * 2 + (mat & 1) < a.ny);
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+              const uint32_t xr = zr ? zrow : xb[d] + (uint32_t)(ks * 2 * WK * XP);
+#pragma unroll
+              for (int n = 0; n < NC / 8; n += 2) {
+                uint32_t b0, b1, b2, b3;
+                ldsm_x4_t(b0, b1, b2, b3, xr + (uint32_t)(n * 16));
+#pragma unroll
+                for (int m = 0; m < MC / 16; ++m) {
+                  mma_bf16(acc[d][m][n], A[m], b0, b1);
+                  mma_bf16(acc[d][m][n + 1], A[m], b2, b3);
+                }
+              }
+            }
+          }
+        };
+        if (part)
+          plane_mma(std::true_type{});
+        else
+          plane_mma(std::false_type{});
+        if (bias && tid < BG * MC) {
+          const __nv_bfloat16 *gp =
+              reinterpret_cast<const __nv_bfloat16 *>(smem + gs * S::GB) + tid % MC;
+          for (int row = tid / MC; row < TK * TJ; row += BG)
+            bsum += __bfloat162float(gp[row * (GP / 2)]);
+        }
+        if (++chain == WG_FLUSH) {
+          chain = 0;
+          flush();
+        }
+      }
+      xs = xs + 1 == XS ? 0 : xs + 1;
+      gs = gs + 1 == GS ? 0 : gs + 1;
+    }
+  }
+  if (chain || !stored) flush();
   if (bias) {
     cp_wait<0>();
     __syncthreads();
@@ -519,37 +620,24 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(float *__restrict__ out
   }
 }
 
-template <int MC, int NC>
-cudaError_t launch_wgrad(float *dw, float *db, const __nv_bfloat16 *g, const __nv_bfloat16 *in,
-                         int nx, int ny, int nz, int cin, int cout, float *ws, int nslots,
+template <int MC, int NC, int ND>
+cudaError_t launch_wgrad(WgArgs a, float *dw, float *db, float *ws, int64_t cap,
                          cudaStream_t s) {
-  constexpr int SMEM = wg_smem_bytes<MC, NC>();
-  if (!smem_opt_in((const void *)conv_wgrad_kernel<MC, NC>, SMEM)) return cudaErrorNotSupported;
-  WgArgs a{};
-  a.g = g;
-  a.in = in;
-  a.nx = nx;
-  a.ny = ny;
-  a.nz = nz;
-  a.cin = cin;
-  a.cout = cout;
-  a.jt = (ny + TJ - 1) / TJ;
-  a.kt = (nz + TK - 1) / TK;
-  a.tiles = (int64_t)nx * a.jt * a.kt;
-  a.nbi = cin / NC;
-  const int blocks = 3 * a.nbi * (cout / MC);
-  // Splits of the voxels: enough CTAs for about three per SM, as many as the
-  // workspace's slots hold (one slot is kept for the bias partials, which fit
-  // it up to 27 cin splits)
+  constexpr int SMEM = WgShape<MC, NC, ND>::SMEM;
+  if (!smem_opt_in((const void *)conv_wgrad_kernel<MC, NC, ND>, SMEM))
+    return cudaErrorNotSupported;
+  a.nbi = a.cin / NC;
+  const int blocks = a.nbi * (a.cout / MC) * (ND == 3 ? 1 : 3);
+  // about three CTAs per SM where the workspace's slots allow as many splits
   const int64_t want = (148 * 3 + blocks - 1) / blocks;
-  int64_t splits = std::min<int64_t>({want, a.tiles, nslots > 1 ? nslots - 1 : 1, 27 * 16});
-  const int64_t n = 27LL * cin * cout;
+  const int64_t splits = std::min<int64_t>({want, a.tiles, cap});
+  const int64_t n = 27LL * a.cin * a.cout;
   float *partb = ws + splits * n;
   a.dst = splits > 1 ? ws : dw;
   a.dbdst = !db ? nullptr : (splits > 1 ? partb : db);
-  conv_wgrad_kernel<MC, NC><<<dim3((unsigned)splits, blocks), WG_THREADS, SMEM, s>>>(a);
+  conv_wgrad_kernel<MC, NC, ND><<<dim3((unsigned)splits, blocks), WG_THREADS, SMEM, s>>>(a);
   if (splits > 1) {
-    const int nb = db ? cout : 0;
+    const int nb = db ? a.cout : 0;
     sum_splits_kernel<<<(unsigned)((n + nb + 31) / 32), 256, 0, s>>>(dw, db, ws, partb,
                                                                      (int)splits, n, nb);
   }
@@ -561,18 +649,6 @@ cudaError_t launch_wgrad(float *dw, float *db, const __nv_bfloat16 *g, const __n
 
 using namespace bsp;
 using namespace bsp::uconv;
-
-namespace bsp {
-// Reads and clears the convolution's give-up flag (bsp_unet_tc_error).
-cudaError_t conv_error_take(int *flag) {
-  cudaError_t e = cudaMemcpyFromSymbol(flag, uconv::g_conv_err, sizeof(int));
-  if (e == cudaSuccess && *flag) {
-    const int zero = 0;
-    e = cudaMemcpyToSymbol(uconv::g_conv_err, &zero, sizeof(int));
-  }
-  return e;
-}
-}  // namespace bsp
 
 extern "C" int bsp_unet_conv3_fwd(bsp_bf16_t *out_, const bsp_bf16_t *in_,
                                   const bsp_bf16_t *w_, const float *bias, int nx, int ny,
@@ -590,42 +666,31 @@ extern "C" int bsp_unet_conv3_fwd(bsp_bf16_t *out_, const bsp_bf16_t *in_,
   a.nx = nx;
   a.ny = ny;
   a.nz = nz;
-  a.cin = cin;
   a.cout = cout;
   a.relu = relu;
-  a.vec = ((uintptr_t)out_ & 15u) == 0;
-  a.cp = cin < CP_MAX ? cin : CP_MAX;
-  a.npass = (cin + CP_MAX - 1) / CP_MAX;
-  // output channels per CTA: the largest tile that divides cout and whose
-  // weights (27 x cp x nt) stay within W_BYTES_MAX
-  a.nt = 64;
-  while (cout % a.nt || a.cp * a.nt > 2048) a.nt >>= 1;
-  a.nct = cout / a.nt;
-  a.wbytes = (27 * a.cp * a.nt * 2 + 127) / 128 * 128;
-  a.slot_bytes = a.cp / 8 * HALF;
-  a.nslot = MAXSLOT;
-  while (a.nslot > 4 && a.wbytes + a.nslot * a.slot_bytes + (int)sizeof(FwdCtl) > SMEM_MAX)
-    --a.nslot;
-  const int smem = a.wbytes + a.nslot * a.slot_bytes + (int)sizeof(FwdCtl);
-  if (smem > SMEM_MAX) return BSP_ERR_SHAPE;
-  a.jt = (ny + TJ - 1) / TJ;
-  a.kt = (nz + TK - 1) / TK;
-  const int64_t cols = (int64_t)a.jt * a.kt * a.nct;
-  // planes per CTA: one wave of CTAs (two per SM when both fit), so that the
-  // weights are loaded and the halo planes re-read as seldom as possible
-  const int occ = smem <= SMEM_MAX / 2 - 1024 ? 2 : 1;
-  int64_t len = (nx * cols + 148 * occ - 1) / (148 * occ);
-  len = std::max<int64_t>(1, std::min<int64_t>(len, nx));
-  a.nacc = 4;
-  if (a.npass > 1) {  // every plane's accumulator stays until the last pass
-    len = std::min<int64_t>(len, MAXACC);
-    a.nacc = MAXACC;
+  const int64_t nvox = (int64_t)nx * ny * nz;
+  // Output channels per CTA: 32 where cout divides by it and 32-channel tiles
+  // still give every SM a CTA, else 16 (at the deepest levels an SM's time is
+  // its weights' load).  128 input channels leave room for 16.
+  const int64_t cells = (int64_t)((ny + TJ - 1) / TJ) * ((nz + TK - 1) / TK) * nx;
+  const bool n32 = cout % 32 == 0 && cells * (cout / 32) >= 148;
+  if ((int64_t)ny * nz * cin < (1 << 30)) {  // offsets inside a plane are 32-bit
+    switch (cin) {
+      case 16: return (int)(n32 ? launch_fwd<16, 32, 2, 3>(a, s) : launch_fwd<16, 16, 2, 3>(a, s));
+      case 32: return (int)(n32 ? launch_fwd<32, 32, 2, 3>(a, s) : launch_fwd<32, 16, 2, 3>(a, s));
+      case 64: return (int)(n32 ? launch_fwd<64, 32, 1, 3>(a, s) : launch_fwd<64, 16, 1, 3>(a, s));
+      case 128: return (int)launch_fwd<128, 16, 1, 2>(a, s);
+      default: break;
+    }
   }
-  a.len = (int)len;
-  const int64_t items = cols * ((nx + len - 1) / len);
-  if (items > 0x7fffffff) return BSP_ERR_SHAPE;
-  if (!smem_opt_in((const void *)conv_fwd_kernel, SMEM_MAX)) return (int)cudaErrorNotSupported;
-  conv_fwd_kernel<<<(unsigned)items, FWD_THREADS, smem, s>>>(a);
+  const int nt = cout % 64 == 0 ? 64 : (cout % 32 == 0 ? 32 : 16);
+  const dim3 grid((unsigned)((nvox + GM - 1) / GM), cout / nt);
+  if (nt == 64)
+    conv_any_kernel<64><<<grid, GM, 0, s>>>(a, cin);
+  else if (nt == 32)
+    conv_any_kernel<32><<<grid, GM, 0, s>>>(a, cin);
+  else
+    conv_any_kernel<16><<<grid, GM, 0, s>>>(a, cin);
   return (int)cudaGetLastError();
 }
 
@@ -648,10 +713,29 @@ extern "C" int bsp_unet_conv3_wgrad(float *dw, float *db, const bsp_bf16_t *g_,
     return BSP_ERR_WORKSPACE;
   if (((uintptr_t)in & 15u) || ((uintptr_t)g & 15u)) return BSP_ERR_ALIGN;
   const int64_t nvox = (int64_t)nx * ny * nz;
-  const int nslots = (int)std::min<int64_t>((nvox + WG_VCH - 1) / WG_VCH, 1 << 30);
-  // channel blocks of 32 where the channels divide by it, else 16
-  const bool m32 = cout % 32 == 0, n32 = cin % 32 == 0;
-  auto fn = m32 ? (n32 ? launch_wgrad<32, 32> : launch_wgrad<32, 16>)
-                : (n32 ? launch_wgrad<16, 32> : launch_wgrad<16, 16>);
-  return (int)fn(dw, db, g, in, nx, ny, nz, cin, cout, workspace, nslots, s);
+  WgArgs a{};
+  a.g = g;
+  a.in = in;
+  a.nx = nx;
+  a.ny = ny;
+  a.nz = nz;
+  a.cin = cin;
+  a.cout = cout;
+  a.jt = (ny + TJ - 1) / TJ;
+  a.kt = (nz + TK - 1) / TK;
+  a.tiles = (int64_t)nx * a.jt * a.kt;
+  // Splits of the voxels: as many as the workspace's slots, less one that is
+  // kept for the bias partials (they fit it up to 27 cin splits).
+  const int64_t nslots = (nvox + WG_VCH - 1) / WG_VCH;
+  const int64_t cap = std::min<int64_t>(std::max<int64_t>(nslots - 1, 1), 27 * 16);
+  // Channel blocks of 32 where the channels divide by it and they still give
+  // two CTAs per SM, else 16; below one CTA per SM each di gets its own.
+  bool m32 = cout % 32 == 0, n32 = cin % 32 == 0;
+  auto ctas = [&]() { return cap * (cout / (m32 ? 32 : 16)) * (cin / (n32 ? 32 : 16)); };
+  if (n32 && ctas() < 2 * 148) n32 = false;
+  if (m32 && ctas() < 2 * 148) m32 = false;
+  if (ctas() < 148) return (int)launch_wgrad<16, 16, 1>(a, dw, db, workspace, cap, s);
+  auto fn = m32 ? (n32 ? launch_wgrad<32, 32, 3> : launch_wgrad<32, 16, 3>)
+                : (n32 ? launch_wgrad<16, 32, 3> : launch_wgrad<16, 16, 3>);
+  return (int)fn(a, dw, db, workspace, cap, s);
 }

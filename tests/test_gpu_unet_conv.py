@@ -13,7 +13,7 @@ from boilingsim_b200._lib import call, ptr
 pytestmark = pytest.mark.gpu
 
 DIMS = [(1, 1, 1), (2, 16, 8), (5, 17, 9), (3, 15, 7), (37, 20, 11), (9, 40, 24)]
-CH = [(16, 16), (32, 64), (128, 32), (80, 48), (16, 160)]
+CH = [(16, 16), (32, 64), (128, 32), (80, 48), (16, 160), (208, 16)]
 
 
 def bf(a):
