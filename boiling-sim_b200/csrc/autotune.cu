@@ -22,7 +22,8 @@ extern int g_sweep_bi, g_sweep_tblock, g_fine_bi;
 extern bool g_coarse_fused_enabled;
 int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                       const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
-                      int n_iter, int tblock, cudaStream_t stream, bool p_zero_nonfluid);
+                      int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero,
+                      unsigned int *bar);
 }  // namespace bsp
 
 namespace {
@@ -71,7 +72,7 @@ extern "C" int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, f
         cudaMemsetAsync(p, 0, bytes, s);
         cudaEventRecord(t.a, s);
         st = jacobi_solve_impl(p, p_tmp, div_u, rhs_ws, mask, nx, ny, nz, dx, dt, rho, sweeps,
-                               0, s, true);
+                               0, s, true, false, nullptr);
         cudaEventRecord(t.b, s);
       }
       if (st == BSP_OK) st = (int)cudaEventSynchronize(t.b);

@@ -17,6 +17,7 @@
 //   * generic kernel: one thread per cell, any shape or alignment.
 // Both produce bit-identical results (same per-cell operation order).
 #include "bsp_common.cuh"
+#include "f32x2.cuh"
 #include "profile.cuh"
 
 namespace bsp {
@@ -320,9 +321,184 @@ __global__ void __launch_bounds__(256) sweep_znf_kernel(float *__restrict__ out,
   }
 }
 
+// ---- point sweep kernel ---------------------------------------------------------
+// The same sweep with one lane per VEC cells of one plane and no march: a thread's
+// loads do not depend on each other (but on the mask, which the launch reads
+// before the sweep ahead of it has finished), so on fields that stay in L2 many
+// short warps hide the latency that a marching warp meets once per plane
+// (192x192x128: 13.4 -> 9.9 us a sweep on a B200; 384x384x256, from HBM: 76
+// against 82, the march stays).  Only fluid cells are read, computed and stored
+// (FILL: +0 stored elsewhere, for a buffer that is not +0 off fluid yet).
+//  VEC = 4 (nz % 4 == 0, 16-byte aligned fields); VEC = 1: any nz, any alignment.
+template <int VEC>
+__device__ __forceinline__ uint32_t ldm(const uint8_t *m) {
+  return VEC == 4 ? __ldg(reinterpret_cast<const uint32_t *>(m)) : (uint32_t)__ldg(m);
+}
+// p: coherent loads (the sweep before may still be writing it when this
+// kernel starts)
+__device__ __forceinline__ Quad ldp(const float *m) {
+  const ulonglong2 t = __ldca(reinterpret_cast<const ulonglong2 *>(m));
+  return Quad{t.x, t.y};
+}
+// v where the neighbour is not solid, ps where it is (v is +0 there); bit 7 of
+// each byte of sw: solid
+__device__ __forceinline__ Quad pick4(uint32_t sw, const Quad &v, const float (&ps)[4]) {
+  float c[4];
+  cells(v, c);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) c[q] = znf_nbr(sw, q, c[q], ps[q]);
+  return quad(c);
+}
+
+template <int VEC, bool FILL>
+__global__ void __launch_bounds__(256, VEC == 4 ? 5 : 6)
+    sweep_point_kernel(float *out, const float *p, const float *__restrict__ rhs,
+                       const uint8_t *__restrict__ mask, int nx, int ny, int nz) {
+  constexpr uint32_t FLUID = VEC == 4 ? 0x80808080u : 0x80u, ONES = FLUID >> 7;
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.y * 8 + (threadIdx.x >> 5), i = blockIdx.z;
+  const int k = (blockIdx.x * 32 + lane) * VEC;
+  const bool act = k < nz && j < ny;
+  const int64_t plane = (int64_t)ny * nz, o = (int64_t)i * plane + (int64_t)j * nz + k;
+  pdl_trigger();
+  const uint32_t mc = act ? ldm<VEC>(mask + o) : 0u;
+  const bool fl = (mc & FLUID) != 0u;
+  if (!__any_sync(0xffffffffu, fl)) {
+    pdl_wait();
+    if (FILL && act) {
+      if constexpr (VEC == 4)
+        *reinterpret_cast<float4 *>(out + o) = make_float4(0.f, 0.f, 0.f, 0.f);
+      else
+        out[o] = 0.0f;
+    }
+    return;
+  }
+  const bool has_jm = j > 0, has_jp = j + 1 < ny, has_im = i > 0, has_ip = i + 1 < nx;
+  // the cell beyond the warp's k range that lanes 0 and 31 need
+  const bool edge = fl && (lane == 0 ? k > 0 : (lane == 31 && k + VEC < nz));
+  const int eoff = lane == 0 ? -1 : VEC;
+  // what stays the same over the solve: rhs, and the neighbours' masks where
+  // some fluid cell has a solid neighbour (mask bits 0-2 count them)
+  const uint32_t cnt = mc & (((mc >> 7) & ONES) * 7u);
+  uint32_t ml = 0, mr = 0, md = 0, mu = 0, me = 0;
+  Quad sv{0, 0};
+  if (fl) {
+    if constexpr (VEC == 4) {
+      const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2 *>(rhs + o));
+      sv = Quad{t.x, t.y};
+    } else {
+      sv.a = __float_as_uint(__ldg(rhs + o));
+    }
+  }
+  const bool solid = __any_sync(0xffffffffu, cnt != 0u);
+  if (solid) {
+    if (cnt) {
+      if (has_im) ml = ldm<VEC>(mask + o - plane);
+      if (has_ip) mr = ldm<VEC>(mask + o + plane);
+      if (has_jm) md = ldm<VEC>(mask + o - nz);
+      if (has_jp) mu = ldm<VEC>(mask + o + nz);
+    }
+    if (edge) me = __ldg(mask + o + eoff);
+  }
+  pdl_wait();
+  Quad c{0, 0}, l{0, 0}, r{0, 0}, d{0, 0}, u{0, 0};
+  float ev = 0.0f;
+  if (fl) {
+    auto ld = [&](int64_t x) {
+      if constexpr (VEC == 4)
+        return ldp(p + x);
+      else
+        return Quad{(uint64_t)__float_as_uint(__ldca(p + x)), 0};
+    };
+    c = ld(o);
+    if (has_im) l = ld(o - plane);
+    if (has_ip) r = ld(o + plane);
+    if (has_jm) d = ld(o - nz);
+    if (has_jp) u = ld(o + nz);
+    if (edge) ev = __ldca(p + o + eoff);
+  }
+  if constexpr (VEC == 4) {
+    float cc[4];
+    cells(c, cc);
+    float km = __shfl_up_sync(0xffffffffu, cc[3], 1), kp = __shfl_down_sync(0xffffffffu, cc[0], 1);
+    if (lane == 0) km = ev;
+    if (lane == 31) kp = ev;
+    float b[4] = {km, cc[0], cc[1], cc[2]}, f[4] = {cc[1], cc[2], cc[3], kp};
+    if (solid) {
+      uint32_t mkm = __shfl_up_sync(0xffffffffu, mc, 1) >> 24;
+      uint32_t mkp = __shfl_down_sync(0xffffffffu, mc, 1);
+      if (lane == 0) mkm = me;
+      if (lane == 31) mkp = me;
+      const uint32_t sb = ((mc << 8) | (mkm & 0xffu)) << 1, sf = ((mc >> 8) | (mkp << 24)) << 1;
+      // a direction without a solid neighbour in the warp keeps its raw values
+      if (__any_sync(0xffffffffu, ((sb | sf) & mc & FLUID) != 0u)) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          b[q] = znf_nbr(sb, q, b[q], cc[q]);
+          f[q] = znf_nbr(sf, q, f[q], cc[q]);
+        }
+      }
+      const uint32_t kc = (((sb >> 7) & ONES) + ((sf >> 7) & ONES)) & (((mc >> 7) & ONES) * 7u);
+      if (__any_sync(0xffffffffu, cnt != kc)) {
+        l = pick4(ml << 1, l, cc);
+        r = pick4(mr << 1, r, cc);
+        d = pick4(md << 1, d, cc);
+        u = pick4(mu << 1, u, cc);
+      }
+    }
+    float t[4];
+    cells(Quad{add2(add2(add2(l.a, r.a), d.a), u.a), add2(add2(add2(l.b, r.b), d.b), u.b)}, t);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t[q] = __fadd_rn(__fadd_rn(t[q], b[q]), f[q]);
+    if (FILL || __any_sync(0xffffffffu, fl && (~mc & FLUID))) {
+      // cells that are not fluid: a quotient away from the division's slow
+      // path, and +0 stored
+      float x[4], y[4];
+      cells(sv, x);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (!(mc >> (8 * q) & BSP_MFLUID)) {
+          x[q] = 1.0f;
+          t[q] = 0.0f;
+        }
+      cells(div6_quad(quad(t), quad(x)), y);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = __uint_as_float(__float_as_uint(y[q]) & fluid_word(mc, q));
+      c = quad(y);
+    } else {
+      c = div6_quad(quad(t), sv);
+    }
+    if (FILL ? act : fl) *reinterpret_cast<ulonglong2 *>(out + o) = make_ulonglong2(c.a, c.b);
+  } else {
+    auto val = [](const Quad &q) { return __uint_as_float((uint32_t)q.a); };
+    const float ps = val(c);
+    float v[6] = {val(l), val(r), val(d), val(u), __shfl_up_sync(0xffffffffu, ps, 1),
+                  __shfl_down_sync(0xffffffffu, ps, 1)};
+    if (lane == 0) v[4] = ev;
+    if (lane == 31) v[5] = ev;
+    if (solid) {
+      uint32_t mkm = __shfl_up_sync(0xffffffffu, mc, 1), mkp = __shfl_down_sync(0xffffffffu, mc, 1);
+      if (lane == 0) mkm = me;
+      if (lane == 31) mkp = me;
+      const uint32_t m[6] = {ml, mr, md, mu, mkm, mkp};
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        if (m[q] & BSP_MSOLID) v[q] = ps;
+    }
+    const float s = __fadd_rn(
+        __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), v[2]), v[3]), v[4]), v[5]);
+    if (fl)
+      out[o] = div6(__fsub_rn(s, val(sv)));
+    else if (FILL && act)
+      out[o] = 0.0f;
+  }
+}
+
 // BSP_TUNE_SWEEP_PREFETCH: the ZNF sweep's L2 prefetch distance in planes
 // (0 off, 2 default, 3).
 int g_sweep_prefetch = 2;
+// Cells up to which a sweep's fields (13 B a cell) count as resident in L2.
+constexpr int64_t L2_SWEEP_CELLS = 10LL << 20;
 
 // ---- generic kernel -----------------------------------------------------------
 template <int OP, class MaskT>
@@ -458,7 +634,7 @@ int g_sweep_bi = 0;
 
 static inline int pick_bi(int nx, int ny, int nz) {
   const int64_t cols = (int64_t)((nz / 4 + 31) / 32) * ((ny + 7) / 8);
-  const int64_t target = (int64_t)num_sms() * 8;
+  const int64_t target = (int64_t)num_sms() * 16;
   int bi = 64;
   while (bi > 4 && cols * ((nx + bi - 1) / bi) < target) bi >>= 1;
   return bi;
@@ -489,14 +665,34 @@ cudaError_t launch_stencil(float *out, const float *p, const float *div, const M
   return cudaGetLastError();
 }
 
-// Jacobi sweep with precomputed rhs on a source whose non-fluid cells are +0
-// (the ZNF column kernel), or the general kernels when the layout does not
-// allow the column kernel.  Bit-identical to launch_stencil<OP_JACOBI_RHS>.
+template <int VEC, bool FILL>
+cudaError_t launch_point(float *out, const float *p, const float *rhs, const uint8_t *mask, int nx,
+                         int ny, int nz, bool pdl, cudaStream_t s) {
+  const dim3 grid((nz + 32 * VEC - 1) / (32 * VEC), (ny + 7) / 8, nx);
+  return launch_maybe_pdl(pdl, grid, dim3(256), 0, s, sweep_point_kernel<VEC, FILL>, out, p, rhs,
+                          mask, nx, ny, nz);
+}
+
+// Jacobi sweep with precomputed rhs on a source whose non-fluid cells are +0.
+// fill: out may hold anything off fluid (it gets +0 there); else out is +0
+// off fluid already.  pdl: the kernel before in the stream is a sweep of the
+// same solve.  Bit-identical to launch_stencil<OP_JACOBI_RHS>.
+// The march (aligned rows only) serves the grids whose fields (13 B a cell) do
+// not stay in L2, and a plane chunk set by the autotuner; the point kernel the
+// rest.  Measured on pots, us a sweep, march / point: 192x192x128 13.4 / 9.9,
+// 384x384x256 76 / 82.
 cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const uint8_t *mask,
-                             int nx, int ny, int nz, cudaStream_t s) {
-  const bool col_ok = (nz % 4 == 0) && aligned16(out) && aligned16(p) && aligned16(rhs) &&
-                      (((uintptr_t)mask & 3u) == 0);
-  if (!col_ok)
+                             int nx, int ny, int nz, bool fill, bool pdl, cudaStream_t s) {
+  const bool vec = (nz % 4 == 0) && aligned16(out) && aligned16(p) && aligned16(rhs) &&
+                   (((uintptr_t)mask & 3u) == 0);
+  const int64_t n = (int64_t)nx * ny * nz;
+  if (nx <= 65535 && (ny + 7) / 8 <= 65535 &&
+      (!vec || (n <= L2_SWEEP_CELLS && g_sweep_bi == 0))) {
+    auto fn = vec ? (fill ? launch_point<4, true> : launch_point<4, false>)
+                  : (fill ? launch_point<1, true> : launch_point<1, false>);
+    return fn(out, p, rhs, mask, nx, ny, nz, pdl, s);
+  }
+  if (!vec)
     return launch_stencil<OP_JACOBI_RHS, uint8_t>(out, p, rhs, mask, nx, ny, nz, 0.f, 1.f, 0.f,
                                                   BSP_FLUID, BSP_AIR, s);
   const int bi = g_sweep_bi > 0 ? g_sweep_bi : pick_bi(nx, ny, nz);

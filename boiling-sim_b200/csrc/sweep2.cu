@@ -223,6 +223,11 @@ __device__ int g_sweep2_err;
 int num_sms();
 extern int g_sweep_bi;  // BSP_TUNE_SWEEP_BI (stencil.cu)
 
+int *sweep2_error_word() {
+  int *err = nullptr;
+  return cudaGetSymbolAddress((void **)&err, g_sweep2_err) == cudaSuccess ? err : nullptr;
+}
+
 // Two sweeps p0 -> out (rhs already hoisted, p0 zero off fluid).  False when
 // the TMA path cannot run (nz % 16 != 0, alignment, no driver entry point).
 bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *mask, int nx,
@@ -235,8 +240,8 @@ bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *
         make_map(&maps.r, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, rhs, nx, ny, nz, FW, R1)))
     return false;
   if (!smem_opt_in((const void *)sweep2_kernel, TOTAL)) return false;
-  int *err = nullptr;
-  if (cudaGetSymbolAddress((void **)&err, g_sweep2_err) != cudaSuccess) return false;
+  int *err = sweep2_error_word();
+  if (!err) return false;
   const int64_t cols = (int64_t)((nz + 127) / 128) * ((ny + ROWS - 1) / ROWS);
   int bi = 16;
   while (bi > 2 && cols * ((nx + bi - 1) / bi) < 2LL * num_sms()) bi -= 2;

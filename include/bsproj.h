@@ -194,15 +194,16 @@ int bsp_jacobi_sweep(float *p_new, const float *p_old, const float *div_u,
  * per-cell constant rho dx^2 div / dt is evaluated into it once and the
  * sweeps read it (bit-identical results, no division per sweep); rhs_ws may
  * equal div_u, which then holds that constant afterwards.  tblock: sweeps
- * per HBM pass -- 0 or 1 (default) one, 2 fuses pairs of sweeps into one
- * temporally blocked pass (needs rhs_ws, nz % 16 == 0 and the source zero
- * off fluid, i.e. from the second sweep, or the first when p starts at
- * zero); the result is bit-identical either way. */
+ * per HBM pass -- 0 or 1 one, 2 fuses pairs of sweeps into one temporally
+ * blocked pass (needs rhs_ws, nz % 16 == 0 and the source zero off fluid, i.e.
+ * from the second sweep, or the first when p starts at zero); the result is
+ * bit-identical either way. */
 int bsp_jacobi_solve(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                      const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
                      int n_iter, int tblock, cudaStream_t stream);
 
-/* 1 in *flag_host if a temporally blocked sweep pass gave up a bounded
+/* 1 in *flag_host if a temporally blocked sweep pass, or a projection whose
+ * sweeps ran in one launch (bsp_projection_jacobi), gave up a bounded
  * device-side wait since the last call (its output is then invalid); clears
  * the flag.  Synchronises the device.  No reference counterpart. */
 int bsp_sweep2_error(int *flag_host);
@@ -250,7 +251,10 @@ int bsp_enforce_no_slip(float *ux, float *uy, float *uz, const uint8_t *mask, in
 
 /* Whole Jacobi projection (fluid.py:612-734): zero p and p_tmp, divergence,
  * n_iter sweeps, gradient subtract, diagnostic divergence.  max|div| after
- * the projection is written to *max_div_dev (device float).  No host sync. */
+ * the projection is written to *max_div_dev (device float).  No host sync.
+ * With tblock 0 and max_div_dev given, grids that fit the SMs' shared memory
+ * (up to about 2 M cells) run their sweeps in one cooperative launch, which
+ * uses *max_div_dev as its barrier word before the diagnostic overwrites it. */
 int bsp_projection_jacobi(float *p, float *p_tmp, float *div_u, float *ux, float *uy,
                           float *uz, const uint8_t *mask, int nx, int ny, int nz, float dx,
                           float dt, float rho, int n_iter, int tblock, float *max_div_dev,
