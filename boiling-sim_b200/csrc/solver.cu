@@ -28,13 +28,16 @@
 #include <cuda_fp16.h>
 
 #include <cstring>
+#include <algorithm>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include <cstddef>
 
 #include "bsp_common.cuh"
 #include "grid_sync.cuh"
+#include "mggroup.cuh"
 #include "profile.cuh"
 #include "solver.cuh"
 
@@ -1274,31 +1277,130 @@ __global__ void __launch_bounds__(RED_THREADS) bnorm_kernel(SolverState *st,
 // level-0 plane chunk in force when it was built is part of its key.
 extern int g_fine_bi;
 struct SetupKey {
-  const void *ws, *mask;
+  const void *mask;
   int nx, ny, nz, storage, fine_bi, tri;  // tri: the parent patterns were built too
   int fine_ctas;                           // tile flags follow the plane chunking
 };
 static std::mutex g_setup_mu;
-static SetupKey g_setups[16];
-static int g_setup_next = 0;
+// by workspace (one setup each); a batch's instances all find theirs again
+static std::unordered_map<const void *, SetupKey> g_setups;
+constexpr size_t SETUPS_MAX = 4096;
 
 static bool setup_cached(const void *ws, const void *mask, int nx, int ny, int nz, int storage) {
   std::lock_guard<std::mutex> lk(g_setup_mu);
-  for (const SetupKey &k : g_setups)
-    if (k.ws == ws && k.mask == mask && k.nx == nx && k.ny == ny && k.nz == nz &&
-        k.storage == storage && k.fine_bi == g_fine_bi && k.tri == (int)g_l0_trilinear &&
-        k.fine_ctas == g_fine_ctas)
-      return true;
-  return false;
+  const auto at = g_setups.find(ws);
+  if (at == g_setups.end()) return false;
+  const SetupKey &k = at->second;
+  return k.mask == mask && k.nx == nx && k.ny == ny && k.nz == nz && k.storage == storage &&
+         k.fine_bi == g_fine_bi && k.tri == (int)g_l0_trilinear && k.fine_ctas == g_fine_ctas;
 }
 static void remember_setup(const void *ws, const void *mask, int nx, int ny, int nz,
                            int storage) {
   std::lock_guard<std::mutex> lk(g_setup_mu);
-  for (SetupKey &k : g_setups)
-    if (k.ws == ws) k.ws = nullptr;  // a workspace holds one setup
-  g_setups[g_setup_next] = SetupKey{ws, mask, nx, ny, nz, storage, g_fine_bi,
-                                     (int)g_l0_trilinear, g_fine_ctas};
-  g_setup_next = (g_setup_next + 1) % 16;
+  if (g_setups.size() >= SETUPS_MAX) g_setups.clear();
+  g_setups[ws] = SetupKey{mask, nx, ny, nz, storage, g_fine_bi, (int)g_l0_trilinear, g_fine_ctas};
+}
+
+// ---- one-launch solve of small grids (mggroup.cu) ---------------------------------
+static_assert(grp::MAXL == MAX_LEVELS && grp::COARSEST == COARSEST_CELLS, "group constants");
+static_assert(4 * grp::PSTRIDE <= 3 * PARTIAL_STRIDE, "the group's sums fit the partials");
+static_assert(sizeof(grp::Result) <= sizeof(SolverState), "the result takes the state's place");
+
+// The line lies where level 1 takes the tile kernels (64-cell rows, 128 K
+// cells: the V-cycle then has two sweeps on it, another method than the group
+// kernel's) and at GROUP_CELLS.  Host-driven, graph and batched solves of a
+// grid all take the same side, so that they agree bit for bit.  The per-kernel
+// path also serves what the group kernel has not: per-kernel tracing, trilinear
+// transfers, the barrier-error test.
+constexpr int64_t GROUP_CELLS = 8LL << 20;
+static bool group_eligible(int nx, int ny, int nz) {
+  if (g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
+  if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
+  const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);
+  if ((nz + 1) / 2 % 4 == 0 && (nz + 1) / 2 >= 64 && n1 >= 131072) return false;
+  int dims[3 * MAX_LEVELS];
+  const int L = build_hierarchy(nx, ny, nz, dims);
+  const int *d = dims + 3 * (L - 1);
+  return (int64_t)d[0] * d[1] * d[2] <= COARSEST_CELLS;
+}
+
+// Waits for an instance's solve and reads its result (its status returned).
+static int group_info(const BspBatchItem &it, int storage, BspSolveInfo *info, cudaStream_t s) {
+  const Layout lo = make_layout(it.nx, it.ny, it.nz, storage);
+  grp::Result r{};
+  cudaError_t e = cudaMemcpyAsync(&r, (char *)it.workspace + lo.state, sizeof(r),
+                                  cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  info->outer_iterations = r.outer_it;
+  info->inner_iterations = r.total_inner;
+  info->rel_residual = r.rel;
+  info->levels = lo.L;
+  return r.status;
+}
+
+// Solves count instances (all eligible, levels set up) in launches of at most
+// GROUP_MAX; infos as in bsp_solve_batch.
+template <class T>
+static int solve_group(int count, const BspBatchItem *items, const BspSolveParams *prm,
+                       BspSolveInfo *infos, cudaStream_t s) {
+  const int most = std::min(grp::GROUP_MAX, num_sms());
+  const int launches = (count + most - 1) / most;
+  for (int b = 0, q0 = 0; b < launches; ++b) {
+    grp::Params P{};
+    P.count = (count - q0 + launches - b - 1) / (launches - b);
+    P.max_outer = prm->max_outer;
+    P.max_inner = prm->max_inner;
+    P.alpha = g_mg_alpha;
+    P.tol = prm->tol;
+    P.eta = prm->inner_tol;
+    P.warm = prm->warm_start && items[q0].p;
+    for (int q = 0; q < P.count; ++q) {
+      const BspBatchItem &it = items[q0 + q];
+      const Layout lo = make_layout(it.nx, it.ny, it.nz, prm->storage);
+      grp::Inst &in = P.in[q];
+      in.base = (char *)it.workspace;
+      in.mask = it.mask;
+      in.div = it.div;
+      in.p = it.p;
+      in.cinv = (const float *)(in.base + lo.cinv);
+      in.cflag = (const int *)(in.base + lo.cflag);
+      in.bscale = -((double)it.rho * (double)it.dx * (double)it.dx) / (double)it.dt;
+      in.nx = it.nx;
+      in.ny = it.ny;
+      in.nz = it.nz;
+      in.L = lo.L;
+      in.off_ctl = lo.cctl;
+      in.off_partials = lo.partials;
+      in.off_result = lo.state;
+      in.off_x = lo.x;
+      in.off_e = lo.e;
+      in.off_z = lo.z;
+      in.off_r = lo.r;
+      in.off_r2 = lo.r2;
+      in.off_ps0 = lo.ps0;
+      in.off_ps1 = lo.ps1;
+      in.off_Ap = lo.Ap;
+      for (int l = 1; l < lo.L; ++l) {
+        in.off_lv[l] = lo.lvl_mask[l];
+        in.off_lr[l] = lo.lvl_r[l];
+        in.off_le[l] = lo.lvl_e[l];
+      }
+      const cudaError_t e = cudaMemsetAsync(in.base + lo.cctl, 0, 64, s);
+      if (e != cudaSuccess) return (int)e;
+    }
+    const cudaError_t e = launch_group_solve<T>(P, s);
+    if (e != cudaSuccess) return (int)e;
+    q0 += P.count;
+  }
+  if (!infos) return BSP_OK;
+  int status = BSP_OK;
+  for (int q = 0; q < count; ++q) {
+    const int st = group_info(items[q], prm->storage, &infos[q], s);
+    if (st != BSP_OK && status == BSP_OK) status = st;
+  }
+  return status;
 }
 
 template <class T>
@@ -1309,6 +1411,16 @@ int solve_impl(void *ws, const uint8_t *mask, const float *div, float *p_out, in
   {
     const Level<T> &c = cx.lv[cx.lo.L - 1];
     if ((int64_t)c.nx * c.ny * c.nz > COARSEST_MAX) return BSP_ERR_SHAPE;
+  }
+  if (group_eligible(nx, ny, nz)) {
+    if (!(prm->reuse_setup && setup_cached(ws, mask, nx, ny, nz, prm->storage))) {
+      const cudaError_t e = setup_levels<T>(cx, s);
+      if (e != cudaSuccess) return (int)e;
+      remember_setup(ws, mask, nx, ny, nz, prm->storage);
+    }
+    const BspBatchItem item{p_out, div, mask, nx, ny, nz, dx, dt, rho, ws, cx.lo.total};
+    BspSolveInfo own{};  // the host-driven solve returns its status even without info
+    return solve_group<T>(1, &item, prm, info ? info : &own, s);
   }
   SolverState h{};
   h.tol = prm->tol;
@@ -1613,6 +1725,8 @@ template <class T>
 int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams *prm,
                       BspSolveInfo *infos, cudaStream_t s) {
   std::vector<Ctx<T>> cxs;
+  // instances for the group kernel, the others for the graph
+  std::vector<int> small_at, large_at;
   GraphKey key;
   key.v.push_back((uintptr_t)count);
   key_params(key, prm);
@@ -1628,11 +1742,23 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
       if (e != cudaSuccess) return (int)e;
       remember_setup(it.workspace, it.mask, it.nx, it.ny, it.nz, prm->storage);
     }
+    if (group_eligible(it.nx, it.ny, it.nz)) {
+      small_at.push_back(q);
+      continue;
+    }
+    large_at.push_back(q);
     for (uintptr_t x : {(uintptr_t)it.workspace, (uintptr_t)it.mask, (uintptr_t)it.div,
                         (uintptr_t)it.p, (uintptr_t)it.nx, (uintptr_t)it.ny, (uintptr_t)it.nz})
       key.v.push_back(x);
     key_floats(key, it.dx, it.dt, it.rho);
     cxs.push_back(cx);
+  }
+  std::vector<BspBatchItem> small;
+  for (int q : small_at) small.push_back(items[q]);
+  if (large_at.empty()) return solve_group<T>(count, small.data(), prm, infos, s);
+  if (!small.empty()) {  // before the graph; their results are read after it
+    const int st = solve_group<T>((int)small.size(), small.data(), prm, nullptr, s);
+    if (st != BSP_OK) return st;
   }
   std::lock_guard<std::mutex> lk(g_graph_mu);
   cudaGraphExec_t exec = graph_lookup(key);
@@ -1640,10 +1766,10 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaGraphCreate(&g, 0);
     prof_suspend(true);
-    for (int q = 0; q < count && e == cudaSuccess; ++q) {
+    for (size_t q = 0; q < large_at.size() && e == cudaSuccess; ++q) {
       std::vector<cudaGraphNode_t> deps;
-      e = append_solve<T>(cxs[q], items[q].div, items[q].p, items[q].dx, items[q].dt,
-                          items[q].rho, prm, g, deps);
+      const BspBatchItem &it = items[large_at[q]];
+      e = append_solve<T>(cxs[q], it.div, it.p, it.dx, it.dt, it.rho, prm, g, deps);
     }
     prof_suspend(false);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
@@ -1656,12 +1782,14 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
   cudaError_t e = cudaGraphLaunch(exec, s);
   if (e != cudaSuccess) return (int)e;
   if (!infos) return BSP_OK;  // asynchronous: results land in p when the stream reaches them
-  int status = BSP_OK;
-  for (int q = 0; q < count; ++q) {
-    const int st = finish_info<T>(cxs[q], &infos[q], s);
-    if (st != BSP_OK && status == BSP_OK) status = st;
-  }
-  return status;
+  std::vector<int> states(count, BSP_OK);
+  for (size_t q = 0; q < large_at.size(); ++q)
+    states[large_at[q]] = finish_info<T>(cxs[q], &infos[large_at[q]], s);
+  for (size_t q = 0; q < small.size(); ++q)
+    states[small_at[q]] = group_info(small[q], prm->storage, &infos[small_at[q]], s);
+  for (int st : states)
+    if (st != BSP_OK) return st;
+  return BSP_OK;
 }
 
 static void key_params(GraphKey &k, const BspSolveParams *p) {
