@@ -779,6 +779,18 @@ struct Layout {
   int L, dims[3 * MAX_LEVELS];
 };
 
+// The group kernel's setup.  Code bytes of level 0 are in eff0 (scratch of the
+// setup, free after it).  In the trilinear patterns' place (the group kernel does
+// not run with those): the list of level-0 units, the coarse levels' code bytes one after the
+// other and (level lo.L) the list's scratch.
+static size_t group_code_offset(const Layout &lo, int l) {
+  if (l == 0) return lo.eff0;
+  size_t off = lo.ppat + al256(4 * (1 + group_units(lo.dims[0], lo.dims[1], lo.dims[2])));
+  for (int m = 1; m < l; ++m)
+    off += (size_t)lo.dims[3 * m] * lo.dims[3 * m + 1] * lo.dims[3 * m + 2];
+  return off;
+}
+
 Layout make_layout(int nx, int ny, int nz, int storage) {
   Layout lo{};
   const size_t n = (size_t)nx * ny * nz, ts = storage_bytes(storage);
@@ -799,8 +811,9 @@ Layout make_layout(int nx, int ny, int nz, int storage) {
   lo.r = take(ts * n);
   lo.r2 = take(ts * n);  // second level-0 residual buffer (fused CG update)
   lo.eff0 = take(n);
-  lo.ppat = take(n);  // level-0 parent patterns of the trilinear transfers
   lo.L = build_hierarchy(nx, ny, nz, lo.dims);
+  lo.ppat = off;  // level-0 parent patterns of the trilinear transfers, or the group kernel's setup
+  take(std::max(n, group_code_offset(lo, lo.L) - lo.ppat + group_units(nx, ny, nz)));
   for (int l = 1; l < lo.L; ++l) {
     const size_t nl = (size_t)lo.dims[3 * l] * lo.dims[3 * l + 1] * lo.dims[3 * l + 2];
     lo.lvl_mask[l] = take(nl);
@@ -891,6 +904,26 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
   return cx;
 }
 
+// The line lies where level 1 takes the tile kernels (64-cell rows, 128 K
+// cells: the V-cycle then has two sweeps on it, another method than the group
+// kernel's, and 192x192x128 FP32 takes 4.2 ms here against 4.4 ms of a group's 200x200x130)
+// and at GROUP_CELLS, the largest size that was measured (331x327x201: 36.4 ms per
+// kernel, 13.5 ms by a group; 384x384x120: 10.7 and 10.5 ms).  Host-driven, graph and
+// batched solves of a grid all take the same side, so that they agree bit for bit.  The
+// per-kernel path also serves what the group kernel has not: per-kernel tracing,
+// trilinear transfers, the barrier-error test.
+constexpr int64_t GROUP_CELLS = 24LL << 20;
+static bool group_eligible(int nx, int ny, int nz) {
+  if (g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
+  if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
+  const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);
+  if ((nz + 1) / 2 % 4 == 0 && (nz + 1) / 2 >= 64 && n1 >= 131072) return false;
+  int dims[3 * MAX_LEVELS];
+  const int L = build_hierarchy(nx, ny, nz, dims);
+  const int *d = dims + 3 * (L - 1);
+  return (int64_t)d[0] * d[1] * d[2] <= COARSEST_CELLS;
+}
+
 template <class T>
 cudaError_t setup_levels(Ctx<T> &cx, cudaStream_t s) {
   // effective classes of level 0 (scratch), then coarsen level by level
@@ -959,6 +992,17 @@ cudaError_t setup_levels(Ctx<T> &cx, cudaStream_t s) {
       coarse_invert_kernel<T><<<1, 1024, 0, s>>>(c, (double *)(cx.base + cx.lo.cA),
                                                  (float *)(cx.base + cx.lo.cinv), flag);
     }
+  }
+  if (group_eligible(cx.nx, cx.ny, cx.nz)) {
+    ProfScope ps(PROF_CONTROL, s);
+    for (int l = 0; l < cx.lo.L; ++l) {
+      const Level<T> &v = cx.lv[l];
+      launch_group_codes((uint8_t *)cx.base + group_code_offset(cx.lo, l), v.mask, v.nx, v.ny,
+                         v.nz, s);
+    }
+    launch_group_units((uint32_t *)(cx.base + cx.lo.ppat),
+                       (uint8_t *)cx.base + group_code_offset(cx.lo, cx.lo.L), cx.lv[0].mask,
+                       cx.nx, cx.ny, cx.nz, s);
   }
   return cudaGetLastError();
 }
@@ -1280,6 +1324,7 @@ struct SetupKey {
   const void *mask;
   int nx, ny, nz, storage, fine_bi, tri;  // tri: the parent patterns were built too
   int fine_ctas;                           // tile flags follow the plane chunking
+  bool group;                              // the group kernel's code bytes were built
 };
 static std::mutex g_setup_mu;
 // by workspace (one setup each); a batch's instances all find theirs again
@@ -1292,37 +1337,21 @@ static bool setup_cached(const void *ws, const void *mask, int nx, int ny, int n
   if (at == g_setups.end()) return false;
   const SetupKey &k = at->second;
   return k.mask == mask && k.nx == nx && k.ny == ny && k.nz == nz && k.storage == storage &&
-         k.fine_bi == g_fine_bi && k.tri == (int)g_l0_trilinear && k.fine_ctas == g_fine_ctas;
+         k.fine_bi == g_fine_bi && k.tri == (int)g_l0_trilinear && k.fine_ctas == g_fine_ctas &&
+         k.group == group_eligible(nx, ny, nz);
 }
 static void remember_setup(const void *ws, const void *mask, int nx, int ny, int nz,
                            int storage) {
   std::lock_guard<std::mutex> lk(g_setup_mu);
   if (g_setups.size() >= SETUPS_MAX) g_setups.clear();
-  g_setups[ws] = SetupKey{mask, nx, ny, nz, storage, g_fine_bi, (int)g_l0_trilinear, g_fine_ctas};
+  g_setups[ws] = SetupKey{mask, nx, ny, nz, storage, g_fine_bi, (int)g_l0_trilinear, g_fine_ctas,
+                           group_eligible(nx, ny, nz)};
 }
 
 // ---- one-launch solve of small grids (mggroup.cu) ---------------------------------
 static_assert(grp::MAXL == MAX_LEVELS && grp::COARSEST == COARSEST_CELLS, "group constants");
 static_assert(4 * grp::PSTRIDE <= 3 * PARTIAL_STRIDE, "the group's sums fit the partials");
 static_assert(sizeof(grp::Result) <= sizeof(SolverState), "the result takes the state's place");
-
-// The line lies where level 1 takes the tile kernels (64-cell rows, 128 K
-// cells: the V-cycle then has two sweeps on it, another method than the group
-// kernel's) and at GROUP_CELLS.  Host-driven, graph and batched solves of a
-// grid all take the same side, so that they agree bit for bit.  The per-kernel
-// path also serves what the group kernel has not: per-kernel tracing, trilinear
-// transfers, the barrier-error test.
-constexpr int64_t GROUP_CELLS = 8LL << 20;
-static bool group_eligible(int nx, int ny, int nz) {
-  if (g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
-  if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
-  const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);
-  if ((nz + 1) / 2 % 4 == 0 && (nz + 1) / 2 >= 64 && n1 >= 131072) return false;
-  int dims[3 * MAX_LEVELS];
-  const int L = build_hierarchy(nx, ny, nz, dims);
-  const int *d = dims + 3 * (L - 1);
-  return (int64_t)d[0] * d[1] * d[2] <= COARSEST_CELLS;
-}
 
 // Waits for an instance's solve and reads its result (its status returned).
 static int group_info(const BspBatchItem &it, int storage, BspSolveInfo *info, cudaStream_t s) {
@@ -1382,10 +1411,16 @@ static int solve_group(int count, const BspBatchItem *items, const BspSolveParam
       in.off_ps0 = lo.ps0;
       in.off_ps1 = lo.ps1;
       in.off_Ap = lo.Ap;
+      in.off_code[0] = lo.eff0;
+      in.units = (const uint32_t *)(in.base + lo.ppat);
+      in.paired0 = it.nz % 4 == 0;
+      in.paired = true;
+      for (int l = 1; l < lo.L; ++l) in.paired &= lo.dims[3 * l + 2] % 4 == 0;
       for (int l = 1; l < lo.L; ++l) {
         in.off_lv[l] = lo.lvl_mask[l];
         in.off_lr[l] = lo.lvl_r[l];
         in.off_le[l] = lo.lvl_e[l];
+        in.off_code[l] = group_code_offset(lo, l);
       }
       const cudaError_t e = cudaMemsetAsync(in.base + lo.cctl, 0, 64, s);
       if (e != cudaSuccess) return (int)e;
