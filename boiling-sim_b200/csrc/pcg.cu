@@ -9,8 +9,10 @@
 // (diag_inverse_apply.cu:44-89).
 //
 // B200 design: the reference issues ~10 launches and a blocking device->host
-// copy per check; here one cooperative launch runs the whole loop.  Each
-// iteration is two grid-wide phases separated by bounded grid barriers:
+// copy per check; here one cooperative launch runs the whole loop.  Grids whose vectors fit
+// on chip (about 2 M cells) are solved by pcgr.cu; this is the streaming form for
+// the others (192x192x128: 36 ms).  Each iteration is two grid-wide phases
+// separated by bounded grid barriers:
 //   A: ps = z + beta ps_prev is formed on the fly (centre and neighbours), the
 //      stencil A ps is applied and stored with ps; partial ps.Ap.
 //   B: p, r, z updated elementwise; partial r.z and r.r.
@@ -18,9 +20,11 @@
 // given grid size).  Vector arithmetic stays FP32 with the reference's
 // expressions (y = fma(a, x, y)).
 // Work unit: one (i, j) row of nz cells per warp, lanes striding over k.
+#include <algorithm>
 #include <type_traits>
 
 #include "grid_sync.cuh"
+#include "pcgr.cuh"
 
 namespace bsp {
 
@@ -448,8 +452,9 @@ static cudaError_t launch_pcg(PcgArgs<MaskT> &a, int max_blocks, cudaStream_t s)
                                      dim3(PCG_THREADS), args, 0, s);
 }
 
-// BSP_TUNE_PCG_QUAD: 1 (default) runs the four-cell form of the PCG phases
-// where it applies, 0 the one-cell form (the same per-cell operations)
+// BSP_TUNE_PCG_QUAD: 1 (default) runs the on-chip form where it fits and else the
+// four-cell form of the PCG phases where it applies, 0 the one-cell form (the same
+// per-cell operations)
 bool g_pcg_quad = true;
 
 // dot_workspace layout (>= 4096 bytes): [0,64) GridCtl, [64, 64 + 8*3*nb) partials
@@ -500,11 +505,29 @@ extern "C" cudaError_t pressure_solve_pcg_launch(
                (uintptr_t)ws_p_search | (uintptr_t)ws_b | (uintptr_t)ws_Ap) & 15u))
                ? 1
                : 0;
-  e = launch_pcg<int32_t>(a, COMPAT_MAX_BLOCKS, 0);
-  if (e != cudaSuccess) return e;
   GridCtl h{};
-  e = cudaMemcpy(&h, ctl, sizeof(GridCtl), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return e;
+  h.status = PR_AGAIN;
+  PcgrPlan plan;
+  if (g_pcg_quad && pcg_resident_fits(nx, ny, nz, std::min(num_sms(), COMPAT_MAX_BLOCKS), plan)) {
+    PcgrArgs r{a.p, a.div, a.mask, a.z, a.partials, a.ctl, {}, nx, ny, nz, a.mf, a.ma, a.max_iter};
+    for (int q = 0; q < 7; ++q) r.outs[q] = dst[q];
+    r.scale = a.scale;
+    r.tol2 = a.tol2;
+    e = launch_pcg_resident(r, plan, 0);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpy(&h, ctl, sizeof(GridCtl), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+    if (h.err == 0 && h.status == PR_AGAIN) {
+      e = cudaMemsetAsync(ctl, 0, sizeof(GridCtl), 0);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  if (h.err == 0 && h.status == PR_AGAIN) {
+    e = launch_pcg<int32_t>(a, COMPAT_MAX_BLOCKS, 0);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpy(&h, ctl, sizeof(GridCtl), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+  }
   if (h.err != 0) return (cudaError_t)h.err;
   if (h.status != 0) return (cudaError_t)h.status;
   if (iter_count_host) *iter_count_host = h.iters;

@@ -75,7 +75,7 @@ extern "C" {
                                      per SM with one each, 0 = per layer (default) */
 #define BSP_TUNE_L1_SWEEPS 17     /* with COARSE_SPLIT: smoothing sweeps a side on level 1, 1 or 2
                                      (default) */
-#define BSP_TUNE_PCG_QUAD 18      /* reference-compatible PCG: four-cell form 1 (default), one-cell 0 */
+#define BSP_TUNE_PCG_QUAD 18      /* reference-compatible PCG: on-chip or four-cell form 1 (default), one-cell 0 */
 #define BSP_TUNE_L0_TRILINEAR 19  /* trilinear transfers between levels 0 and 1: 1 on, 0 off */
 #define BSP_TUNE_TRI_CPC 20       /* coarse planes per thread of the trilinear restriction (1..64) */
 #define BSP_TUNE_FUSE_SCALARS 21  /* CG scalars in the last CTA of the level-0 kernels: 1, 0 (default) */
