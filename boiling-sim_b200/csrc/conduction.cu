@@ -35,8 +35,12 @@
 // T on every cell once and stores it to T_old, replacing the separate copy.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/bsproj.h"
+#include "blocks.cuh"
 #include "bsp_common.cuh"
+#include "grid_sync.cuh"
 #include "tma.cuh"
 
 namespace bsp {
@@ -376,7 +380,7 @@ __global__ void cls_assign_kernel(uint8_t *__restrict__ cls, uint32_t *__restric
 }
 
 // Per-CTA class table: tab[2c] = (1 + sum gamma, g-x, g+x, g-y), tab[2c+1] =
-// (g+y, g-z, g+z, 0).  gamma of a material pair as in gamma_entry; EDGE and
+// (g+y, g-z, g+z, 1 / (1 + sum gamma)).  gamma of a material pair as in gamma_entry; EDGE and
 // ids >= n_mat give 0.  Class 0 (air) gets den 1 and zero gammas.
 __device__ __forceinline__ void build_class_table(float4 *tab, float *gt,
                                                   const uint32_t *__restrict__ patterns, int ncls,
@@ -398,7 +402,7 @@ __device__ __forceinline__ void build_class_table(float4 *tab, float *gt,
       }
     }
     tab[2 * c] = make_float4(__fadd_rn(1.0f, diag), g[0], g[1], g[2]);
-    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], 0.0f);
+    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], __fdiv_rn(1.0f, __fadd_rn(1.0f, diag)));
   }
   __syncthreads();
 }
@@ -421,6 +425,17 @@ __device__ __forceinline__ bool cls_some(uint32_t w) {
   return (w & 0x80808080u) != 0x80808080u;
 }
 __device__ __forceinline__ bool cls_every(uint32_t w) { return (w & 0x80808080u) == 0u; }
+
+// a / d, correctly rounded, with y = 1 / d correctly rounded: after one step the
+// quotient is within a unit in the last place, and a step from there rounds as a
+// division does (Markstein) -- as long as nothing leaves the normal range, else
+// the division itself.
+__device__ __forceinline__ float div_by(float a, float d, float y) {
+  float q = __fmul_rn(a, y);
+  if (!(fabsf(q) > 1e-30f && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
+  q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+}
 
 // One cell of class c: rhs over the faces -x, +x, -y, +y, -z, +z in order.
 __device__ __forceinline__ float be_cell(const float4 *tab, uint32_t c, float tm, float tp,
@@ -861,6 +876,303 @@ int sweep(float *T_dst, const float *T_iter, const float *T_old, const MatT *mat
   return (int)launch_sweep<MatT, false>(T_dst, T_iter, T_old, nullptr, mat, nx, ny, nz, P, s);
 }
 
+// ---- sweeps on chip ------------------------------------------------------------------
+// On a small grid a sweep is a launch whose CTAs each build the class table and
+// march a few planes: 12.9 us at 110x110x68.  Here one cooperative launch runs all sweeps
+// of a step: a CTA keeps a block of columns and its halo in shared memory (two
+// iterates, air at T_amb and 0 outside the grid, so a cell's six values are plain loads),
+// works on a list of its cells that are not air (T_old in registers), and only
+// the cells at a block's sides go through memory, into the array that the sweep would have
+// written; a barrier between sweeps.  The same operations on every cell.  Measured:
+// 193 -> 79 us for 15 sweeps at 110x110x68, 819 -> 340 us for 50 at 140x140x96.
+// The barrier's words take the place of T_old's first two cells, which the last CTA
+// to leave writes; T and T_alt end up as after the sweeps one by one (their last two
+// iterates; after an odd number T takes T_alt's air cells too, as the copy does).
+namespace res {
+constexpr int THREADS = 1024, WARPS = 32;
+constexpr int SLOTS = 16;                  // cells a thread, at most
+constexpr int COLS = 256;                  // columns of a block (list entry)
+constexpr int SMEM = 227 * 1024 - 12288;   // dynamic shared memory a CTA may take
+// list entry: place | class << 16 | side << 23 | column << 24
+constexpr uint32_t SIDE = 1u << 23;
+
+struct Args {
+  float *T, *Ta, *To;
+  const void *mat;  // class bytes, or material ids
+  const uint32_t *patterns;
+  unsigned int *bar;  // arrivals, leavers
+  int *err;
+  int ncls, nx, ny, nz, nbx, nby, pad, cap, cols, n_iter;
+  Params P;
+};
+
+// A face's code in a key of material ids: the neighbour's id, 15 on the domain edge
+// (no gamma).  Ids are masked as by the kernels that take such a grid's sweeps one by one.
+template <class MatT>
+__device__ __forceinline__ uint32_t id_key(const MatT *m, int c, int i, int j, int k, int nx,
+                                           int ny, int nz) {
+  const uint32_t mask = nz % 4 == 0 ? TCOLS - 1 : MAXM - 1;
+  auto code = [&](bool in, int off) { return in ? mbyte(m, c + off) & mask : (uint32_t)OOB; };
+  return code(i > 0, -ny * nz) | code(i + 1 < nx, ny * nz) << 4 | code(j > 0, -nz) << 8 |
+         code(j + 1 < ny, nz) << 12 | code(k > 0, -1) << 16 | code(k + 1 < nz, 1) << 20 |
+         (mbyte(m, c) & (MAXM - 1)) << 24;
+}
+
+// CLS: mat holds class bytes; else material ids, with each listed cell's key beside
+// its entry (geometries of more than 127 classes).
+template <class MatT, bool CLS>
+__global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_constant__ Args a) {
+  extern __shared__ float cr_smem[];
+  __shared__ float4 tab[2 * NCLS];
+  __shared__ float gt[MAXM * TCOLS];
+  __shared__ int wcount[WARPS], s_ok;
+  float *P0 = cr_smem, *P1 = P0 + a.pad;                   // iterates of the block and its halo
+  uint32_t *E = reinterpret_cast<uint32_t *>(P1 + a.pad);  // cells that are not air
+  int *gp = reinterpret_cast<int *>(E + a.cap);            // column -> cell - place
+  uint32_t *HM = reinterpret_cast<uint32_t *>(gp + a.cols);  // halo, 32 k cells each: not air
+  int2 *H;                                                   // its first cell and place
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int bi = blockIdx.x / a.nby, bj = blockIdx.x - bi * a.nby;
+  const int i0 = (int)((int64_t)nx * bi / a.nbx), i1 = (int)((int64_t)nx * (bi + 1) / a.nbx);
+  const int j0 = (int)((int64_t)ny * bj / a.nby), j1 = (int)((int64_t)ny * (bj + 1) / a.nby);
+  const int w = i1 - i0, h = j1 - j0, ncol = w * h, cells = ncol * nz;
+  const int dk = nz + 2, di = (h + 2) * dk;  // strides of the iterates along j, i
+  const int hcols = 2 * (w + h), ch = (nz + 31) / 32, halo = hcols * ch;
+  H = reinterpret_cast<int2 *>(HM + ((a.cap + a.cols + halo) & 1) + halo);  // on 8 bytes
+  uint32_t *K = reinterpret_cast<uint32_t *>(H + halo);                     // keys of the list
+  const MatT *mat = static_cast<const MatT *>(a.mat);
+  const float tamb = a.P.tamb;
+  const uint32_t mair = (uint32_t)a.P.mair;
+  auto is_air = [&](int c) { return CLS ? (mbyte(mat, c) & CLS_AIR) != 0 : mbyte(mat, c) == mair; };
+  if (CLS)
+    build_class_table(tab, gt, a.patterns, a.ncls, a.P);
+  else
+    build_table16(gt, a.P);
+  float t01[2] = {0.0f, 0.0f};
+  if (tid == 0) {
+    s_ok = 1;
+    t01[0] = a.T[0];
+    t01[1] = a.T[1];
+  }
+  for (int c = tid; c < ncol; c += THREADS) {
+    const int li = c / h, lj = c - li * h;
+    gp[c] = ((i0 + li) * ny + j0 + lj) * nz - ((li + 1) * di + (lj + 1) * dk + 1);
+  }
+  for (int c = tid; c < (w + 2) * di; c += THREADS) P0[c] = P1[c] = 0.0f;
+  __syncthreads();
+
+  // ---- the list, T_old, and the first iterate with air at T_amb -----------------------
+  for (int n = warp; n < halo; n += WARPS) {
+    const int hc = n / ch, k = (n - hc * ch) * 32;
+    int li, lj;
+    if (hc < h) li = -1, lj = hc;
+    else if (hc < 2 * h) li = w, lj = hc - h;
+    else if (hc < 2 * h + w) li = hc - 2 * h, lj = -1;
+    else li = hc - 2 * h - w, lj = h;
+    const int i = i0 + li, j = j0 + lj, at = (li + 1) * di + (lj + 1) * dk + 1 + k;
+    const int c = (i * ny + j) * nz + k;
+    const bool in = i >= 0 && i < nx && j >= 0 && j < ny && k + lane < nz;
+    const bool air = in && is_air(c + lane);
+    if (in) P0[at + lane] = air ? tamb : a.T[c + lane];
+    if (air) P1[at + lane] = tamb;
+    const uint32_t m = __ballot_sync(0xffffffffu, in && !air);
+    if (lane == 0) {
+      H[n] = make_int2(c, at);
+      HM[n] = m;
+    }
+  }
+  int nc = 0;
+  for (int base = 0; base < cells; base += THREADS) {
+    const int l = base + tid;
+    bool live = false;
+    uint32_t entry = 0, key = 0;
+    if (l < cells) {
+      const int col = l / nz, k = l - col * nz, li = col / h, lj = col - li * h;
+      const int at = (li + 1) * di + (lj + 1) * dk + 1 + k, c = gp[col] + at;
+      const float t = a.T[c];
+      live = !is_air(c);
+      if (!CLS && live) key = id_key(mat, c, i0 + li, j0 + lj, k, nx, ny, nz);
+      P0[at] = live ? t : tamb;
+      if (!live) P1[at] = tamb;
+      if (c > 1) a.To[c] = t;
+      const bool side = li == 0 || li + 1 == w || lj == 0 || lj + 1 == h;
+      entry = (uint32_t)at | (CLS ? mbyte(mat, c) << 16 : 0u) | (side ? SIDE : 0u) |
+              (uint32_t)col << 24;
+    }
+    const unsigned int vote = __ballot_sync(0xffffffffu, live);
+    if (lane == 0) wcount[warp] = __popc(vote);
+    __syncthreads();
+    const int n = wcount[lane];
+    int x = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const int before = __shfl_sync(0xffffffffu, x - n, warp);
+    if (live) {
+      const int at = nc + before + __popc(vote & ((1u << lane) - 1u));
+      E[at] = entry;
+      if (!CLS) K[at] = key;
+    }
+    nc += __shfl_sync(0xffffffffu, x, 31);
+    __syncthreads();
+  }
+  float to[SLOTS];
+#pragma unroll
+  for (int q = 0; q < SLOTS; ++q) {
+    const int t = q * THREADS + tid;
+    to[q] = t < nc ? P0[E[t] & 0xffffu] : 0.0f;
+  }
+
+  unsigned int epoch = 0;
+  auto barrier = [&]() {  // arrivals on a counter that only grows; bounded
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned int target = ++epoch * gridDim.x;
+      cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(a.bar[0]);
+      cuda::atomic_ref<int, cuda::thread_scope_device> err(*a.err);
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      cnt.fetch_add(1u, cuda::memory_order_relaxed);
+      unsigned int spins = 0;
+      unsigned long long t0 = 0;
+      while (cnt.load(cuda::memory_order_acquire) < target) {
+        if ((++spins & 255u) == 0) {
+          const unsigned long long now = gs_global_ns();
+          if (t0 == 0) t0 = now;
+          if (now - t0 > BAR_TIMEOUT_NS || spins > BAR_SPIN_LIMIT) {
+            err.store(1, cuda::memory_order_relaxed);
+            s_ok = 0;
+            break;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    return s_ok != 0;
+  };
+
+  // ---- sweeps --------------------------------------------------------------------------
+  const float *cur = P0;
+  float *nxt = P1;
+  for (int s = 1;; ++s) {
+    float *dst = (s & 1) ? a.Ta : a.T;
+    const bool last = s == a.n_iter;
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+      const int t = q * THREADS + tid;
+      if (q * THREADS >= nc) break;
+      if (t < nc) {
+        const uint32_t e = E[t];
+        const int at = (int)(e & 0xffffu), cl = (int)((e >> 16) & 127u);
+        const float *p = cur + at;
+        float v;
+        if (CLS) {
+          const float4 A = tab[2 * cl], B = tab[2 * cl + 1];
+          float rhs = __fadd_rn(0.0f, __fmul_rn(A.y, p[-di]));
+          rhs = __fadd_rn(rhs, __fmul_rn(A.z, p[di]));
+          rhs = __fadd_rn(rhs, __fmul_rn(A.w, p[-dk]));
+          rhs = __fadd_rn(rhs, __fmul_rn(B.x, p[dk]));
+          rhs = __fadd_rn(rhs, __fmul_rn(B.y, p[-1]));
+          rhs = __fadd_rn(rhs, __fmul_rn(B.z, p[1]));
+          v = div_by(__fadd_rn(to[q], rhs), A.x, B.w);
+        } else {
+          const uint32_t key = K[t];
+          const float *row = gt + (key >> 24) * TCOLS;
+          float rhs = 0.0f, diag = 0.0f;
+          face_t(rhs, diag, row, key, 0, p[-di]);
+          face_t(rhs, diag, row, key >> 4, 0, p[di]);
+          face_t(rhs, diag, row, key >> 8, 0, p[-dk]);
+          face_t(rhs, diag, row, key >> 12, 0, p[dk]);
+          face_t(rhs, diag, row, key >> 16, 0, p[-1]);
+          face_t(rhs, diag, row, key >> 20, 0, p[1]);
+          v = __fdiv_rn(__fadd_rn(to[q], rhs), __fadd_rn(1.0f, diag));
+        }
+        nxt[at] = v;
+        if (!last && (e & SIDE)) __stcg(dst + gp[e >> 24] + at, v);
+      }
+    }
+    if (last) break;
+    if (!barrier()) return;
+    constexpr int HQ = 4;  // loads in flight
+    for (int n0 = warp; n0 < halo; n0 += HQ * WARPS) {
+      float v[HQ];
+      int at[HQ];
+#pragma unroll
+      for (int m = 0; m < HQ; ++m) {
+        const int n = n0 + m * WARPS;
+        const bool in = n < halo && ((HM[n] >> lane) & 1u);
+        const int2 x = n < halo ? H[n] : make_int2(0, 0);
+        at[m] = in ? x.y + lane : -1;
+        v[m] = in ? __ldcg(dst + x.x + lane) : 0.0f;
+      }
+#pragma unroll
+      for (int m = 0; m < HQ; ++m)
+        if (at[m] >= 0) nxt[at[m]] = v[m];
+    }
+    __syncthreads();
+    float *t = const_cast<float *>(cur);
+    cur = nxt;
+    nxt = t;
+  }
+
+  // ---- the last two iterates -----------------------------------------------------------
+  // Odd: a CTA may still read the sides of iterate n - 1 in T.
+  const bool odd = a.n_iter & 1;
+  if (odd && !barrier()) return;
+  for (int t = tid; t < nc; t += THREADS) {
+    const int at = (int)(E[t] & 0xffffu), c = gp[E[t] >> 24] + at;
+    a.T[c] = nxt[at];
+    a.Ta[c] = odd ? nxt[at] : cur[at];
+  }
+  if (odd)
+    for (int l = tid; l < cells; l += THREADS) {
+      const int col = l / nz, li = col / h, lj = col - li * h;
+      const int c = gp[col] + (li + 1) * di + (lj + 1) * dk + 1 + (l - col * nz);
+      if (is_air(c)) a.T[c] = a.Ta[c];
+    }
+  if (tid == 0) {
+    // every CTA is past its last poll of the words when the last one is here
+    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> left(a.bar[1]);
+    if (left.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
+      a.To[0] = t01[0];
+      a.To[1] = t01[1];
+    }
+  }
+}
+
+// True when the sweeps have been launched.  A block's cells all need a slot (what is air is
+// known on the device only): up to about 2 M cells.  Two sweeps cost less one by one at
+// the larger of these sizes (140x140x96: 33 us, 39 us here; 56x56x40: 20 and 15 us), three
+// do not (110x110x68: 43 us, 33 us here).
+constexpr int MIN_ITER = 3;
+template <class MatT, bool CLS>
+bool launch(float *T, float *Ta, float *To, const MatT *mat, const uint32_t *patterns, int ncls,
+            int nx, int ny, int nz, const Params &P, int n_iter, cudaStream_t s) {
+  if (n_iter < MIN_ITER || nz < 2 || (int64_t)nx * ny * nz > (int64_t)SLOTS * THREADS * num_sms())
+    return false;
+  const BlockSplit b = split_blocks(nx, ny, num_sms());
+  const int64_t pad = (int64_t)(b.w + 2) * (b.h + 2) * (nz + 2);
+  const int64_t cells = (int64_t)b.w * b.h * nz, halo = 2LL * (b.w + b.h) * ((nz + 31) / 32);
+  const int64_t bytes = 4 * (2 * pad + (CLS ? 1 : 2) * cells + b.w * b.h + 1 + 3 * halo);
+  if (b.w * b.h > COLS || pad > (1 << 16) || cells > SLOTS * THREADS || bytes > SMEM) return false;
+  int *err = nullptr;
+  if (cudaGetSymbolAddress((void **)&err, g_cond_err) != cudaSuccess) return false;
+  Args a{T, Ta, To, mat, patterns, reinterpret_cast<unsigned int *>(To), err, ncls, nx, ny, nz,
+         b.nbx, b.nby, (int)pad, (int)cells, b.w * b.h, n_iter, P};
+  const void *kernel = (const void *)be_resident_kernel<MatT, CLS>;
+  if (!smem_opt_in(kernel, SMEM)) return false;
+  if (cudaMemsetAsync(To, 0, 2 * sizeof(unsigned int), s) != cudaSuccess) return false;
+  void *args[] = {&a};
+  if (cudaLaunchCooperativeKernel(kernel, dim3(b.nbx * b.nby), dim3(THREADS), args, (size_t)bytes,
+                                  s) == cudaSuccess)
+    return true;
+  (void)cudaGetLastError();
+  return false;
+}
+}  // namespace res
+
 // The conduction step: T_old <- T (fused into the first sweep), n_iter sweeps
 // T -> T_alt -> T ..., and T <- T_alt when n_iter is odd.  With n_iter == 0 the
 // step is the snapshot alone.
@@ -877,6 +1189,8 @@ int be_step(float *T, float *T_alt, float *T_old, const MatT *mat, int nx, int n
   const Params P{k, rho, cp, n_mat, dx, dt, h, tamb, mair};
   if (n_iter == 0)
     return (int)cudaMemcpyAsync(T_old, T, bytes, cudaMemcpyDeviceToDevice, s);
+  if (res::launch<MatT, false>(T, T_alt, T_old, mat, nullptr, 0, nx, ny, nz, P, n_iter, s))
+    return BSP_OK;
   cudaError_t e = launch_sweep<MatT, true>(T_alt, T, nullptr, T_old, mat, nx, ny, nz, P, s);
   for (int it = 1; it < n_iter && e == cudaSuccess; ++it) {
     const float *src = (it % 2 == 0) ? T : T_alt;
@@ -1088,6 +1402,9 @@ extern "C" int bsp_conduction_be_cls(float *T, float *T_alt, float *T_old, const
   const size_t bytes = sizeof(float) * (size_t)nx * ny * nz;
   const Params P{k, rho, cp, n_mat, dx, dt, h_conv_air, T_amb, mat_air};
   if (n_iter == 0) return (int)cudaMemcpyAsync(T_old, T, bytes, cudaMemcpyDeviceToDevice, s);
+  if (res::launch<uint8_t, true>(T, T_alt, T_old, cls, patterns, n_classes, nx, ny, nz, P, n_iter,
+                                 s))
+    return BSP_OK;
   cudaError_t e = launch_cls_sweep<true>(T_alt, T, nullptr, T_old, cls, patterns, n_classes,
                                          tiles, nx, ny, nz, P, s);
   for (int it = 1; it < n_iter && e == cudaSuccess; ++it) {

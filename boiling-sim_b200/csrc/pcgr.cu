@@ -17,6 +17,7 @@
 // grid size.
 #include <algorithm>
 
+#include "blocks.cuh"
 #include "grid_sync.cuh"
 #include "pcgr.cuh"
 
@@ -119,7 +120,8 @@ __device__ __forceinline__ float pr_dinv(const PrSync &s, float r, uint32_t e) {
   return __fmaf_rn(__fmaf_rn(-q, d.x, r), d.y, q);
 }
 
-__global__ void __launch_bounds__(PR_THREADS, 1) pcg_resident_kernel(const __grid_constant__ PcgrArgs a) {
+__global__ void __launch_bounds__(PR_THREADS, 1)
+    pcg_resident_kernel(const __grid_constant__ PcgrArgs a) {
   extern __shared__ float pr_smem[];
   __shared__ PrSync s;
   __shared__ int wcount[PR_WARPS + 1];
@@ -361,30 +363,19 @@ __global__ void __launch_bounds__(PR_THREADS, 1) pcg_resident_kernel(const __gri
   }
 }
 
-// Blocks for the grid: the split into at most `ctas` with the fewest cells (a halo cell
-// counted as half) in its largest block.  Taken where the largest block's padded
-// search direction leaves slots for 2/5 of its cells: the pots' fluid is half of
-// their cells, and a block in the middle of one is nearly all fluid below the water
-// line.  What does not fit is known only after the list is made (a few tens of
-// microseconds of a solve of milliseconds) and solved by the streaming form.
+// Taken where the largest block's padded search direction leaves slots for 2/5 of
+// its cells: the pots' fluid is half of their cells, and a block in the middle of one
+// is nearly all fluid below the water line.  What does not fit is known only
+// after the list is made (a few tens of microseconds of a solve of milliseconds)
+// and solved by the streaming form.
 bool pcg_resident_fits(int nx, int ny, int nz, int ctas, PcgrPlan &plan) {
   const int64_t n = (int64_t)nx * ny * nz;
   if (n > (1 << 28)) return false;
   ctas = std::min(ctas, 160);
-  double best = 1e30;
-  int w = 0, h = 0;
-  for (int x = 1; x <= std::min(nx, ctas); ++x) {
-    const int y = std::min(ny, ctas / x);
-    const int bw = (nx + x - 1) / x, bh = (ny + y - 1) / y;
-    const double cost = (double)bw * bh + (bw + bh);
-    if (cost < best) {
-      best = cost;
-      plan.nbx = x;
-      plan.nby = y;
-      w = bw;
-      h = bh;
-    }
-  }
+  const BlockSplit b = split_blocks(nx, ny, ctas);
+  plan.nbx = b.nbx;
+  plan.nby = b.nby;
+  const int w = b.w, h = b.h;
   const int64_t pad = (int64_t)(w + 2) * (h + 2) * (nz + 2);
   if ((int64_t)w * h > PR_COLS || pad > (1 << 16)) return false;
   plan.cols = w * h;
