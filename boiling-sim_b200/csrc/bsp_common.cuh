@@ -163,4 +163,15 @@ inline bool smem_opt_in(const void *fn, int bytes) {
   return ok;
 }
 
+// a / d, correctly rounded, with y = 1 / d correctly rounded: after one step the
+// quotient is within a unit in the last place, and a step from there rounds as a
+// division does (Markstein) -- as long as nothing leaves the normal range, else
+// the division itself.
+__device__ __forceinline__ float div_by(float a, float d, float y) {
+  float q = __fmul_rn(a, y);
+  if (!(fabsf(q) > 1e-30f && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
+  q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+}
+
 }  // namespace bsp

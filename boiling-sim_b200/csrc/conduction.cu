@@ -426,17 +426,6 @@ __device__ __forceinline__ bool cls_some(uint32_t w) {
 }
 __device__ __forceinline__ bool cls_every(uint32_t w) { return (w & 0x80808080u) == 0u; }
 
-// a / d, correctly rounded, with y = 1 / d correctly rounded: after one step the
-// quotient is within a unit in the last place, and a step from there rounds as a
-// division does (Markstein) -- as long as nothing leaves the normal range, else
-// the division itself.
-__device__ __forceinline__ float div_by(float a, float d, float y) {
-  float q = __fmul_rn(a, y);
-  if (!(fabsf(q) > 1e-30f && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
-  q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
-  return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
-}
-
 // One cell of class c: rhs over the faces -x, +x, -y, +y, -z, +z in order.
 __device__ __forceinline__ float be_cell(const float4 *tab, uint32_t c, float tm, float tp,
                                          float tjm, float tjp, float tkm, float tkp, float to) {
