@@ -19,7 +19,8 @@
 //
 // The cycle, the smoother, the stopping tests, the storage and the order of the
 // floating-point operations on every cell are the per-kernel path's with one sweep a
-// side on every level; only sums over cells are taken in another order (in FP64).  Every
+// side on every level (a grid of rows of no whole quads gets that path's bits, others agree
+// to the last places); only sums over cells are taken in another order (in FP64).  Every
 // such sum is taken over a fixed number of virtual warps and then over those in a
 // fixed order, so a result does not depend on how many CTAs its group has:
 // single, batched, host-driven and device-driven solves agree bit for bit.
@@ -772,7 +773,8 @@ __global__ void __launch_bounds__(THREADS, 1) group_solve_kernel(const __grid_co
       lv[l].ny = y;
       lv[l].nz = z;
       lv[l].code = reinterpret_cast<const uint8_t *>(g.in.base + g.in.off_code[l]);
-      lv[l].mask = l == 0 ? g.in.mask : reinterpret_cast<const uint8_t *>(g.in.base + g.in.off_lv[l]);
+      lv[l].mask =
+          l == 0 ? g.in.mask : reinterpret_cast<const uint8_t *>(g.in.base + g.in.off_lv[l]);
       lv[l].r = reinterpret_cast<T *>(g.in.base + (l == 0 ? g.in.off_r : g.in.off_lr[l]));
       lv[l].e = reinterpret_cast<T *>(g.in.base + (l == 0 ? g.in.off_z : g.in.off_le[l]));
       x = (x + 1) / 2;
@@ -898,7 +900,8 @@ __global__ void __launch_bounds__(THREADS, 1) group_solve_kernel(const __grid_co
     if (lost) break;
     const double inv = 1.0 / scale;
     for (int c = t0; c < n; c += tstep)
-      if (__ldg(lv[0].code + c) & FLUID) x[c] += (double)fmaf((float)alpha, ld(last, c), e[c]) * inv;
+      if (__ldg(lv[0].code + c) & FLUID)
+        x[c] += (double)fmaf((float)alpha, ld(last, c), e[c]) * inv;
     xzero = false;
     if (!barrier(g)) { lost = true; break; }
   }
