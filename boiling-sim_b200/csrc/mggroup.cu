@@ -210,10 +210,9 @@ __device__ __forceinline__ Seg seg_of(const Fine &d, uint32_t u) {
 }
 // Neighbour sum of the operand values (0 off fluid), a solid neighbour counting as
 // the cell itself; the k neighbours are the lanes beside.  Two orders, the ones the
-// per-kernel path sums in, so that a grid's vectors (in 16 bits a last place is
-// 5e-4 of a value) are the same on either path: paired with n_solid x centre added
-// (rows of whole quads), or one after the other with the centre in a solid
-// neighbour's place (code bits 0-5).
+// per-kernel path sums in (in 16 bits a last place is 5e-4 of a value): paired with n_solid
+// x centre added (rows of whole quads), or one after the other with the centre in a
+// solid neighbour's place (code bits 0-5).
 __device__ __forceinline__ float six(float l, float r, float d, float u, float b, float f) {
   return ((l + r) + (d + u)) + (b + f);
 }
