@@ -19,11 +19,13 @@
 //
 // The cycle, the smoother, the stopping tests, the storage and the order of the
 // floating-point operations on every cell are the per-kernel path's with one sweep a
-// side on every level (a grid of rows of no whole quads gets that path's bits, others agree
-// to the last places); only sums over cells are taken in another order (in FP64).  Every
-// such sum is taken over a fixed number of virtual warps and then over those in a
-// fixed order, so a result does not depend on how many CTAs its group has:
-// single, batched, host-driven and device-driven solves agree bit for bit.
+// side on every level, to the four-cell FP32 chains of its dots: 16-bit directions turn
+// a last place of alpha or beta into another iterate within the tolerance.  Only the FP64 sums
+// of those chains are taken in another order, far below a place of the FP32 scalars made
+// from them, so the results are that path's bits.  Every such sum is taken over a fixed
+// number of virtual warps and then over those in a fixed order, so a result does not depend on how
+// many CTAs its group has: single, batched, host-driven and device-driven solves agree
+// bit for bit.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -45,6 +47,7 @@ namespace grp {
 constexpr int THREADS = 1024, WARPS = THREADS / 32;
 constexpr int VB = 148;             // virtual blocks of a sum
 constexpr int KOUT = 30;            // k cells of a unit
+constexpr int KQUADS = 28;          // of a level-0 unit on rows of whole quads: whole quads
 constexpr float W = 6.0f / 7.0f;    // smoothing weight
 constexpr float W_C = 1.0f - W;
 constexpr int SEG = 4;              // j values of a level-0 unit
@@ -176,10 +179,11 @@ __device__ __forceinline__ void publish(Ctx<T> &g, int q) {
 // with the next step's loads in flight: two values formed a cell instead of the five of
 // a cell by itself.  Only units with fluid are dealt out.
 struct Fine {
-  int nx, ny, nz, segs, ch;
+  int nx, ny, nz, segs, ch, kout;
 };
 __host__ __device__ __forceinline__ Fine fine_of(int nx, int ny, int nz) {
-  return Fine{nx, ny, nz, (ny + SEG - 1) / SEG, (nz + KOUT - 1) / KOUT};
+  const int kout = nz % 4 == 0 ? KQUADS : KOUT;
+  return Fine{nx, ny, nz, (ny + SEG - 1) / SEG, (nz + kout - 1) / kout, kout};
 }
 struct Seg {
   int i, j0, j1, k, c;      // c: cell (i, j0, k), k clamped into the grid
@@ -195,7 +199,7 @@ __device__ __forceinline__ Seg seg_of(const Fine &d, uint32_t u) {
   t.i = 2 * bi;
   t.j0 = (r - bi * d.segs) * SEG;
   t.j1 = min(t.j0 + SEG, d.ny);
-  t.k = c * KOUT - 1 + lane;
+  t.k = c * d.kout - 1 + lane;
   const bool in = t.k >= 0 && t.k < d.nz, b = t.i + 1 < d.nx, l = t.i > 0, rr = t.i + 2 < d.nx;
   t.c = (t.i * d.ny + t.j0) * d.nz + min(max(t.k, 0), d.nz - 1);
   t.ob = b ? pl : 0;
@@ -205,7 +209,7 @@ __device__ __forceinline__ Seg seg_of(const Fine &d, uint32_t u) {
   t.mb = b ? t.ma : 0u;
   t.ml = l ? t.ma : 0u;
   t.mr = rr ? t.ma : 0u;
-  t.out = in && lane >= 1 && lane <= KOUT;
+  t.out = in && lane >= 1 && lane <= d.kout;
   return t;
 }
 // Neighbour sum of the operand values (0 off fluid), a solid neighbour counting as
@@ -231,6 +235,18 @@ __device__ __forceinline__ float nsum(const float *ns, uint32_t code, float c, f
   }
   return l + r + d + u + b + f;
 }
+// A thread's products of a dot, for its FP64 sum.  PAIRED, as the per-kernel path's
+// four-cell chains: the four cells of a quad in one chain of FP32 FMAs along k (each
+// lane takes the chain over from the lane before; the quad's last cell adds it).
+// Otherwise each product by itself in FP64.  x, y: 0 where the cell does not count.
+template <bool PAIRED>
+__device__ __forceinline__ double prod(float x, float y, int k) {
+  if constexpr (!PAIRED) return (double)x * (double)y;
+  float v = __fmul_rn(x, y);  // of the quad's first cell
+#pragma unroll
+  for (int q = 1; q < 4; ++q) v = fmaf(x, y, __shfl_up_sync(0xffffffffu, v, 1));
+  return (k & 3) == 3 ? (double)v : 0.0;
+}
 // Sum of a coarse cell's children: columns (i, j), (i, j + 1), (i + 1, j),
 // (i + 1, j + 1), each the lane's k and the next lane's; in the per-kernel path's order
 // (level 0 by rows, or child after child).
@@ -241,6 +257,10 @@ __device__ __forceinline__ float children(float a, float a1, float b, float b1) 
   if constexpr (PAIRED) return ((a + an) + (b + bn)) + ((a1 + a1n) + (b1 + b1n));
   return a + an + a1 + a1n + b + bn + b1 + b1n;
 }
+
+// An operand that is a product is rounded by itself (__fmul_rn), as the per-kernel path
+// stores it: contracted into the neighbour sum, it took the restricted residual, and
+// with it z, off that path's by last places.
 
 // The march's loads carry no predicates: addresses outside the grid are
 // clamped to a cell of it, and what such a lane, column or row may not add is
@@ -283,11 +303,11 @@ __device__ __noinline__ void down0(Ctx<T> &g, const LevelP<T> &f, const LevelP<T
       const Centre m = centre(t.j0 > 0 ? c - nz : c), now = centre(c);
       Centre up = centre(t.j0 + 1 < d.ny ? c + nz : c);
       Outer side = outer(c);
-      float am = t.j0 > 0 ? res(m.ra, m.pa) * g.wt[m.ka & t.ma] : 0.0f;
-      float bm = t.j0 > 0 ? res(m.rb, m.pb) * g.wt[m.kb & t.mb] : 0.0f;
+      float am = t.j0 > 0 ? __fmul_rn(res(m.ra, m.pa), g.wt[m.ka & t.ma]) : 0.0f;
+      float bm = t.j0 > 0 ? __fmul_rn(res(m.rb, m.pb), g.wt[m.kb & t.mb]) : 0.0f;
       float ra = res(now.ra, now.pa), rb = res(now.rb, now.pb);
       uint32_t ka = now.ka & t.ma, kb = now.kb & t.mb;
-      float a = ra * g.wt[ka], b = rb * g.wt[kb], ya1 = 0.0f, yb1 = 0.0f;
+      float a = __fmul_rn(ra, g.wt[ka]), b = __fmul_rn(rb, g.wt[kb]), ya1 = 0.0f, yb1 = 0.0f;
 #pragma unroll 1
       for (int j = t.j0; j < t.j1; ++j, c += nz) {
         Centre up2 = up;
@@ -299,21 +319,17 @@ __device__ __noinline__ void down0(Ctx<T> &g, const LevelP<T> &f, const LevelP<T
         const uint32_t row = j + 1 < d.ny ? 0xffu : 0u;
         const uint32_t kau = up.ka & t.ma & row, kbu = up.kb & t.mb & row;
         const float rau = res(up.ra, up.pa), rbu = res(up.rb, up.pb);
-        const float au = rau * g.wt[kau], bu = rbu * g.wt[kbu];
-        const float l = res(side.rl, side.pl) * g.wt[side.kl & t.ml];
-        const float r = res(side.rr, side.pr) * g.wt[side.kr & t.mr];
+        const float au = __fmul_rn(rau, g.wt[kau]), bu = __fmul_rn(rbu, g.wt[kbu]);
+        const float l = __fmul_rn(res(side.rl, side.pl), g.wt[side.kl & t.ml]);
+        const float r = __fmul_rn(res(side.rr, side.pr), g.wt[side.kr & t.mr]);
         const bool oa = t.out && (ka & FLUID), ob = t.out && (kb & FLUID);
         const float sa = nsum<PAIRED>(g.ns, ka, a, l, b, am, au);
         const float sb = nsum<PAIRED>(g.ns, kb, b, a, r, bm, bu);
-        const float ya = oa ? ra - (6.0f * a - sa) : 0.0f, yb = ob ? rb - (6.0f * b - sb) : 0.0f;
-        if (oa) {
-          stv(r_out, c, ra);
-          rr += (double)ra * (double)ra;
-        }
-        if (ob) {
-          stv(r_out, c + t.ob, rb);
-          rr += (double)rb * (double)rb;
-        }
+        const float ya = oa ? ra - fmaf(6.0f, a, -sa) : 0.0f, yb = ob ? rb - fmaf(6.0f, b, -sb) : 0.0f;
+        if (oa) stv(r_out, c, ra);
+        if (ob) stv(r_out, c + t.ob, rb);
+        const float xa = oa ? ra : 0.0f, xb = ob ? rb : 0.0f;
+        rr += prod<PAIRED>(xa, xa, t.k) + prod<PAIRED>(xb, xb, t.k);
         if ((j & 1) || j + 1 == d.ny) {
           const bool odd = j & 1;
           const float acc = children<PAIRED>(odd ? ya1 : ya, odd ? ya : 0.0f, odd ? yb1 : yb,
@@ -378,7 +394,7 @@ __device__ __noinline__ void up0(Ctx<T> &g, const LevelP<T> &f, const LevelP<T> 
                                __shfl_down_sync(0xffffffffu, e, 1));
           return w > 0.0f ? fmaf(w, v + s6, W_C * e) : e;
         }
-        return fmaf(v - (6.0f * e - nsum<false>(g.ns, k, e, l, r1, dn, u)), w, e);
+        return fmaf(v - fmaf(6.0f, e, -nsum<false>(g.ns, k, e, l, r1, dn, u)), w, e);
       };
       int c = t.c;
       const int jm = t.j0 > 0 ? -1 : 0, jp = t.j0 + 1 < d.ny ? 1 : 0;
@@ -406,14 +422,11 @@ __device__ __noinline__ void up0(Ctx<T> &g, const LevelP<T> &f, const LevelP<T> 
         const float r1 = hat(side.kr & t.mr, side.pr, side.rr);
         const float ya = smooth(ka, ra, a, l, b, am, au);
         const float yb = smooth(kb, rb, b, a, r1, bm, bu);
-        if (t.out && (ka & FLUID)) {
-          stv(out, c, ya);
-          rz += (double)ra * (double)rnd(ya, out);
-        }
-        if (t.out && (kb & FLUID)) {
-          stv(out, c + t.ob, yb);
-          rz += (double)rb * (double)rnd(yb, out);
-        }
+        const bool oa = t.out && (ka & FLUID), ob = t.out && (kb & FLUID);
+        if (oa) stv(out, c, ya);
+        if (ob) stv(out, c + t.ob, yb);
+        rz += prod<PAIRED>(oa ? ra : 0.0f, oa ? rnd(ya, out) : 0.0f, t.k) +
+              prod<PAIRED>(ob ? rb : 0.0f, ob ? rnd(yb, out) : 0.0f, t.k);
         am = a, bm = b, a = au, b = bu, ka = kau, kb = kbu;
         ra = ld(&up.ra, 0), rb = ld(&up.rb, 0);
         up = up2;
@@ -477,20 +490,20 @@ __device__ __noinline__ void direction(Ctx<T> &g, const LevelP<T> &f, const T *z
         const float l = dir(t.ml, side.zl, side.pl), r = dir(t.mr, side.zr, side.pr);
         const float sa = nsum<PAIRED>(g.ns, side.ka, a, l, b, am, au);
         const float sb = nsum<PAIRED>(g.ns, side.kb, b, a, r, bm, bu);
-        if (t.out && (side.ka & FLUID)) {
-          const float ap = rnd(6.0f * a - sa, Ap);
+        const bool oa = t.out && (side.ka & FLUID), ob = t.out && (side.kb & t.mb & FLUID);
+        const float apa = oa ? rnd(fmaf(6.0f, a, -sa), Ap) : 0.0f;
+        const float apb = ob ? rnd(fmaf(6.0f, b, -sb), Ap) : 0.0f;
+        if (oa) {
           stv(cur, c, a);
           e[c] = fmaf(alpha, ld(&pa, 0), ea);
-          stv(Ap, c, ap);
-          pap += (double)a * (double)ap;
+          stv(Ap, c, apa);
         }
-        if (t.out && (side.kb & t.mb & FLUID)) {
-          const float ap = rnd(6.0f * b - sb, Ap);
+        if (ob) {
           stv(cur, c + t.ob, b);
           e[c + t.ob] = fmaf(alpha, ld(&pb, 0), eb);
-          stv(Ap, c + t.ob, ap);
-          pap += (double)b * (double)ap;
+          stv(Ap, c + t.ob, apb);
         }
+        pap += prod<PAIRED>(oa ? a : 0.0f, apa, t.k) + prod<PAIRED>(ob ? b : 0.0f, apb, t.k);
         am = a, bm = b, a = au, b = bu, pa = up.pa, pb = up.pb;
         up = up2;
         side = side2;
@@ -557,11 +570,12 @@ __device__ __noinline__ void down(Ctx<T> &g, const LevelP<T> &f, const LevelP<T>
     const int C = (I * co.ny + J) * co.nz + (k >> 1);
     const bool emit = q == 0 && !(k & 1) && k >= 0 && k < nz && lane >= 1 && lane <= KOUT;
     const uint32_t mc = emit ? (uint32_t)__ldg(co.code + C) : 0u;
-    const float y = ld(&v.c, 0), c = y * g.wt[m.c];
-    const float s = nsum<PAIRED>(g.ns, m.c, c, ld(&v.l, 0) * g.wt[m.l], ld(&v.r, 0) * g.wt[m.r],
-                         ld(&v.d, 0) * g.wt[m.d], ld(&v.u, 0) * g.wt[m.u]);
+    auto pre = [&](const T &r, uint32_t n) { return __fmul_rn(ld(&r, 0), g.wt[n]); };
+    const float y = ld(&v.c, 0), c = pre(v.c, m.c);
+    const float s = nsum<PAIRED>(g.ns, m.c, c, pre(v.l, m.l), pre(v.r, m.r), pre(v.d, m.d),
+                                 pre(v.u, m.u));
     float *part = g.part + flip;
-    part[threadIdx.x] = x.out && (m.c & FLUID) ? y - (6.0f * c - s) : 0.0f;
+    part[threadIdx.x] = x.out && (m.c & FLUID) ? y - fmaf(6.0f, c, -s) : 0.0f;
     asm volatile("bar.sync %0, 128;" ::"r"(quad + 1) : "memory");
     if (q == 0) {
       const float *p = part + threadIdx.x;
@@ -598,12 +612,13 @@ __device__ __noinline__ void up(Ctx<T> &g, const LevelP<T> &f, const LevelP<T> &
     const float y = ld(&v.c, 0), c = hat(m.c, p.c, v.c);
     const float s = nsum<PAIRED>(g.ns, m.c, c, hat(m.l, p.l, v.l),
                          hat(m.r, p.r, v.r), hat(m.d, p.d, v.d), hat(m.u, p.u, v.u));
-    if (x.out && (m.c & FLUID)) stv(f.e, x.c, fmaf(y - (6.0f * c - s), g.wt[m.c], c));
+    if (x.out && (m.c & FLUID)) stv(f.e, x.c, fmaf(y - fmaf(6.0f, c, -s), g.wt[m.c], c));
   }
 }
 
 // FP64 residual b - A x on level 0.  WRITE: rhat = scale r (stored as T), e = 0;
-// else the sum of squares and the largest |r|.  ZERO: x is zero.
+// else the sum of squares and the largest |r|.  zero: x is zero.  The neighbours are
+// summed in the per-kernel path's orders, as in nsum (quads: paired).
 template <class T, bool WRITE>
 __device__ void residual(Ctx<T> &g, const LevelP<T> &f, const double *x, T *rhat, float *e,
                          double scale, bool zero) {
@@ -615,18 +630,24 @@ __device__ void residual(Ctx<T> &g, const LevelP<T> &f, const double *x, T *rhat
     for (int c = (vb * WARPS + warp) * 32 + lane; c < n; c += VB * THREADS) {
       const uint32_t m = __ldg(f.code + c);
       if (!(m & FLUID)) continue;
-      double r = g.in.bscale * (double)__ldg(g.in.div + c);
+      const double b = (double)__ldg(g.in.div + c);
+      double ax = 0.0;
       if (!zero) {
         const int t = c / nz, k = c - t * nz, i = t / ny, j = t - i * ny;
         const double xc = x[c];
-        // 0 off fluid; a solid neighbour gives the cell's own value
-        auto nbx = [&](bool in, uint32_t bit, int off) {
-          return m & bit ? xc : (in ? x[c + off] : 0.0);
-        };
-        const double s = nbx(i > 0, 1u, -pl) + nbx(i + 1 < f.nx, 2u, pl) + nbx(j > 0, 4u, -nz) +
-                         nbx(j + 1 < ny, 8u, nz) + nbx(k > 0, 16u, -1) + nbx(k + 1 < nz, 32u, 1);
-        r -= 6.0 * xc - s;
+        auto at = [&](bool in, int off) { return in ? x[c + off] : 0.0; };  // 0 off fluid
+        const double l = at(i > 0, -pl), r1 = at(i + 1 < f.nx, pl), d = at(j > 0, -nz);
+        const double u = at(j + 1 < ny, nz), k0 = at(k > 0, -1), k1 = at(k + 1 < nz, 1);
+        double s;
+        if (g.in.quads) {
+          s = fma((double)__popc(m & SOLIDS), xc, ((l + r1) + (d + u)) + (k0 + k1));
+        } else {  // a solid neighbour gives the cell's own value
+          auto own = [&](uint32_t bit, double v) { return m & bit ? xc : v; };
+          s = own(1u, l) + own(2u, r1) + own(4u, d) + own(8u, u) + own(16u, k0) + own(32u, k1);
+        }
+        ax = fma(6.0, xc, -s);
       }
+      const double r = fma(g.in.bscale, b, -ax);
       if (WRITE) {
         stv(rhat, c, (float)(r * scale));
         e[c] = 0.0f;
@@ -729,11 +750,18 @@ __device__ void coarsest(Ctx<T> &g, const LevelP<T> &L) {
           auto nbe = [&](bool in, int off) {
             if (!in) return 0.0f;
             const uint32_t mn = __ldg(L.mask + t + off);
-            return (mn & BSP_MFLUID) ? a[t + off] : ((mn & BSP_MSOLID) ? ec : 0.0f);
+            return (mn & BSP_MFLUID) ? a[t + off] : ((mn & BSP_MSOLID) && !g.in.paired ? ec : 0.0f);
           };
-          const float sum = nbe(i > 0, -pl) + nbe(i + 1 < L.nx, pl) + nbe(j > 0, -L.nz) +
-                            nbe(j + 1 < L.ny, L.nz) + nbe(k > 0, -1) + nbe(k + 1 < L.nz, 1);
-          v = ec + (g.rr[t] - (6.0f * ec - sum)) / (6.0f - (float)(m & 7u));
+          const float l = nbe(i > 0, -pl), r = nbe(i + 1 < L.nx, pl), d = nbe(j > 0, -L.nz);
+          const float u = nbe(j + 1 < L.ny, L.nz), bk = nbe(k > 0, -1), f = nbe(k + 1 < L.nz, 1);
+          if (g.in.paired) {  // damped; nbe of a solid is then 0 and the centre added after
+            const float n = (float)(m & 7u), w = 6.0f - n;
+            const float sum = fmaf(n, ec, six(l, r, d, u, bk, f));
+            v = fmaf(g.rr[t] - fmaf(6.0f, ec, -sum), w > 0.0f ? __fdividef(W, w) : 0.0f, ec);
+          } else {
+            const float sum = l + r + d + u + bk + f;
+            v = ec + (g.rr[t] - fmaf(6.0f, ec, -sum)) / (6.0f - (float)(m & 7u));
+          }
         }
         b[t] = v;
       }

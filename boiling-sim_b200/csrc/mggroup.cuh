@@ -32,7 +32,9 @@ struct Inst {
   const uint32_t *units;  // level-0 units with fluid: their number, then their list
   double bscale;
   int nx, ny, nz, L;
-  bool paired0, paired;  // order of the neighbour sums: level 0, coarse levels
+  // which of the per-kernel path's orders of operations: level 0 on whole quads, its FP64
+  // residual too, the coarse levels as the one-launch cycle
+  bool paired0, quads, paired;
   int cta0, ncta;  // first CTA of the group, CTAs
   size_t off_ctl, off_partials, off_result, off_x, off_e, off_z, off_r, off_r2, off_ps0, off_ps1,
       off_Ap;

@@ -87,6 +87,8 @@ extern int g_cluster_tail_cells;  // BSP_TUNE_CLUSTER_TAIL_CELLS (mgcoarse.cu)
 extern int g_downu_blocks;        // BSP_TUNE_DOWNU_BLOCKS (mgfine.cu)
 extern bool g_coarse_cluster_tail_smem;  // BSP_TUNE_CLUSTER_TAIL (mgcoarse.cu)
 extern int g_tri_cpc;  // BSP_TUNE_TRI_CPC (mgfine.cu)
+// BSP_TUNE_GROUP_SOLVE: small grids by the one-launch solve (mggroup.cu)
+bool g_group_solve = true;
 // BSP_TUNE_FUSE_UPDATE: CG update fused into the next level-0 restriction
 bool g_fuse_update_enabled = true;
 // BSP_TUNE_TEST_BARRIER_ERROR (tests only): the next host-driven solve starts
@@ -861,6 +863,21 @@ struct Ctx {
   T *r_write() const { return fuse ? (T *)(base + lo.r2) : lv[0].r; }  // rhat target
 };
 
+// Level 0 on the column kernels (mgfine.cu).
+static bool column_layout(int nx, int ny, int nz, const uint8_t *mask) {
+  return nz % 4 == 0 && ((uintptr_t)mask & 15u) == 0 && g_fine_col_enabled &&
+         fine_grid_blocks(nx, ny, nz) <= PARTIAL_STRIDE;
+}
+// A coarse level that the column kernels take too: only while a row keeps at least 16
+// lanes busy (8 from level 3 with BSP_TUNE_COARSE_SPLIT = 3, which takes it onto the
+// tile kernels).
+static bool column_level(int l, int nx, int ny, int nz) {
+  const bool deep = g_coarse_split >= 3 && l >= 3;
+  return g_fine_col_enabled && nz % 4 == 0 && nz >= (deep ? 32 : 64) &&
+         (int64_t)nx * ny * nz >= (deep ? 32768 : 131072) &&
+         fine_grid_blocks(nx, ny, nz) <= PARTIAL_STRIDE;
+}
+
 template <class T>
 Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int storage) {
   Ctx<T> cx{};
@@ -873,8 +890,7 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
   cx.nz = nz;
   cx.n = (int64_t)nx * ny * nz;
   cx.mask0 = mask;
-  cx.col = (nz % 4 == 0) && (((uintptr_t)mask & 15u) == 0) && g_fine_col_enabled &&
-           fine_grid_blocks(nx, ny, nz) <= PARTIAL_STRIDE;
+  cx.col = column_layout(nx, ny, nz, mask);
   cx.fuse = cx.col && g_fuse_update_enabled && fine_tma_available(nz);
   for (int l = 0; l < cx.lo.L; ++l) {
     Level<T> &L = cx.lv[l];
@@ -904,9 +920,9 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
   return cx;
 }
 
-// The line lies where level 1 takes the tile kernels (64-cell rows, 128 K
-// cells: the V-cycle then has two sweeps on it, another method than the group
-// kernel's, and 192x192x128 FP32 takes 4.2 ms here against 4.4 ms of a group's 200x200x130)
+// The line lies where a coarse level takes the column kernels (level 1: 64-cell rows, 128 K
+// cells; the V-cycle then has two sweeps on it and sums in their order, another method than the
+// group kernel's, and 192x192x128 FP32 takes 4.2 ms there against 4.4 ms of a group's 200x200x130)
 // and at GROUP_CELLS, the largest size that was measured (331x327x201: 36.4 ms per
 // kernel, 13.5 ms by a group; 384x384x120: 10.7 and 10.5 ms).  Host-driven, graph and
 // batched solves of a grid all take the same side, so that they agree bit for bit.  The
@@ -914,13 +930,15 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
 // trilinear transfers, the barrier-error test.
 constexpr int64_t GROUP_CELLS = 24LL << 20;
 static bool group_eligible(int nx, int ny, int nz) {
-  if (g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
+  if (!g_group_solve || g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
   if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
   const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);
   if ((nz + 1) / 2 % 4 == 0 && (nz + 1) / 2 >= 64 && n1 >= 131072) return false;
   int dims[3 * MAX_LEVELS];
   const int L = build_hierarchy(nx, ny, nz, dims);
   const int *d = dims + 3 * (L - 1);
+  for (int l = 1; l < L; ++l)
+    if (column_level(l, dims[3 * l], dims[3 * l + 1], dims[3 * l + 2])) return false;
   return (int64_t)d[0] * d[1] * d[2] <= COARSEST_CELLS;
 }
 
@@ -1015,14 +1033,7 @@ cudaError_t launch_inner_iteration(Ctx<T> &cx, int it_parity, cudaStream_t s) {
   const bool col = cx.col;
   auto level_col = [&](int l) {
     const Level<T> &v = cx.lv[l];
-    if (l == 0) return col;
-    // coarse levels: only while a row keeps at least 16 lanes busy (8 on
-    // level 3 with BSP_TUNE_COARSE_SPLIT = 3, which takes it onto the tile
-    // kernels)
-    const bool deep = g_coarse_split >= 3 && l >= 3;
-    return g_fine_col_enabled && v.nz % 4 == 0 && v.nz >= (deep ? 32 : 64) &&
-           (int64_t)v.nx * v.ny * v.nz >= (deep ? 32768 : 131072) &&
-           fine_grid_blocks(v.nx, v.ny, v.nz) <= PARTIAL_STRIDE;
+    return l == 0 ? col : column_level(l, v.nx, v.ny, v.nz);
   };
   // V-cycle on r -> z: level-0 restriction, the coarse levels (one
   // cooperative kernel, or one kernel per level and direction), level-0
@@ -1413,8 +1424,9 @@ static int solve_group(int count, const BspBatchItem *items, const BspSolveParam
       in.off_Ap = lo.Ap;
       in.off_code[0] = lo.eff0;
       in.units = (const uint32_t *)(in.base + lo.ppat);
-      in.paired0 = it.nz % 4 == 0;
-      in.paired = true;
+      in.paired0 = column_layout(it.nx, it.ny, it.nz, it.mask);
+      in.quads = in.paired0 && ((uintptr_t)it.div & 15u) == 0;
+      in.paired = g_coarse_fused_enabled;
       for (int l = 1; l < lo.L; ++l) in.paired &= lo.dims[3 * l + 2] % 4 == 0;
       for (int l = 1; l < lo.L; ++l) {
         in.off_lv[l] = lo.lvl_mask[l];

@@ -861,6 +861,7 @@ extern int g_tri_cpc;
 extern bool g_fuse_scalars;
 extern int g_fine_ctas;
 extern bool g_pdl;
+extern bool g_group_solve;
 extern int g_coarse_cluster;
 extern int g_cluster_tail_cells;
 extern int g_downu_blocks;
@@ -939,6 +940,10 @@ extern "C" int bsp_set_tuning(int key, int value) {
     case BSP_TUNE_COARSE_CLUSTER:
       if (value != 0 && (value < 2 || value > 16)) return BSP_ERR_ARG;
       bsp::g_coarse_cluster = value;
+      return BSP_OK;
+    case BSP_TUNE_GROUP_SOLVE:
+      if (value < 0 || value > 1) return BSP_ERR_ARG;
+      bsp::g_group_solve = value != 0;
       return BSP_OK;
     case BSP_TUNE_PDL:
       if (value < 0 || value > 1) return BSP_ERR_ARG;

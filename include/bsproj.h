@@ -93,6 +93,8 @@ extern "C" {
                                           run in its CTA 0 alone (default 16384) */
 #define BSP_TUNE_DOWNU_BLOCKS 28  /* CTAs per SM of the fused CG update + restriction: 3 (default)
                                      or 4 (48 registers a thread) */
+#define BSP_TUNE_GROUP_SOLVE 29   /* to-tolerance solves of small grids in one launch: 1 on (default),
+                                     0 off (the same bits) */
 
 /* ------------------------------------------------------------------ */
 /* 1. reference-compatible launchers                                   */
