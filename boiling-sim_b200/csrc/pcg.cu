@@ -291,13 +291,13 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_persistent_kernel(PcgArgs<Mas
         v[1] += (double)b * (double)z;
       }
     }
-    block_partials<2>(v, a.partials, a.stride, sh);
+    block_partials<2>(v, a.partials + PCG_SUM_INIT * a.stride, a.stride, sh);
   }
   if (!grid_barrier(a.ctl)) return;
-  double tot[3];
+  double tot[2];
   {
     double t2[2];
-    grid_totals<2>(a.partials, a.stride, t2, sh);
+    grid_totals<2>(a.partials + PCG_SUM_INIT * a.stride, a.stride, t2, sh);
     tot[0] = t2[0];
     tot[1] = t2[1];
   }
@@ -362,12 +362,12 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_persistent_kernel(PcgArgs<Mas
             v[0] += (double)psc * (double)ap;
           }
         }
-        block_partials<1>(v, a.partials, a.stride, sh);
+        block_partials<1>(v, a.partials + PCG_SUM_A * a.stride, a.stride, sh);
       }
       if (!grid_barrier(a.ctl)) return;
       {
         double t1[1];
-        grid_totals<1>(a.partials, a.stride, t1, sh);
+        grid_totals<1>(a.partials + PCG_SUM_A * a.stride, a.stride, t1, sh);
         pAp = t1[0];
       }
       alpha = (pAp == 0.0) ? 0.0 : rz / pAp;
@@ -404,12 +404,12 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_persistent_kernel(PcgArgs<Mas
             v[1] += (double)rc * (double)rc;
           }
         }
-        block_partials<2>(v, a.partials + a.stride, a.stride, sh);
+        block_partials<2>(v, a.partials + PCG_SUM_B * a.stride, a.stride, sh);
       }
       if (!grid_barrier(a.ctl)) return;
       {
         double t2[2];
-        grid_totals<2>(a.partials + a.stride, a.stride, t2, sh);
+        grid_totals<2>(a.partials + PCG_SUM_B * a.stride, a.stride, t2, sh);
         rz_new = t2[0];
         rsq = t2[1];
       }

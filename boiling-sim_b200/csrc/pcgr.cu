@@ -34,8 +34,8 @@ constexpr int PR_SMEM = 227 * 1024 - 4096;    // dynamic shared memory a CTA may
 constexpr uint32_t PR_SIDE = 1u << 22;
 
 struct PrSync {
-  double red[3][PR_WARPS];  // of the CTA's warps
-  double tot[3];
+  double red[2][PR_WARPS];  // of the CTA's warps
+  double tot[2];
   unsigned int epoch;       // barriers passed
   int ok;
   float2 dinv[64];          // by solid bits: D and 1 / D
@@ -222,7 +222,9 @@ __global__ void __launch_bounds__(PR_THREADS, 1)
 
   // ---- z = D^-1 b, p = 0 -----------------------------------------------------------
   float X[PR_SLOTS], p[PR_SLOTS];  // X: z, and A ps between the phases
-  double v[3] = {0.0, 0.0, over && tid == 0 ? 1.0 : 0.0};
+  double v[2] = {0.0, 0.0};
+  // cleared by the host before the launch, read after the barrier
+  if (over && tid == 0) __stcg(&a.ctl->status, PR_AGAIN);
 #pragma unroll
   for (int q = 0; q < PR_SLOTS; ++q) {
     const int t = q * PR_THREADS + tid;
@@ -237,11 +239,9 @@ __global__ void __launch_bounds__(PR_THREADS, 1)
       v[1] += (double)b * (double)X[q];
     }
   }
-  if (!pr_barrier<3>(s, a, v, a.partials)) return;
-  if (v[2] > 0.0) {  // the same in every CTA
-    if (blockIdx.x == 0 && tid == 0) a.ctl->status = PR_AGAIN;
-    return;
-  }
+  if (!pr_barrier<2>(s, a, v, a.partials + PCG_SUM_INIT * gridDim.x)) return;
+  // the same in every CTA (nothing else that is ever written there is PR_AGAIN)
+  if (__ldcg(&a.ctl->status) == PR_AGAIN) return;
   const double bsq = v[0];
   double rz = v[1];
   double alpha = 0.0, beta = 0.0, rz_new = 0.0, rsq = bsq, pAp = 0.0;
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1)
             d[0] += (double)c * (double)X[q];
           }
         }
-        if (!pr_barrier<1>(s, a, d, a.partials)) return;
+        if (!pr_barrier<1>(s, a, d, a.partials + PCG_SUM_A * gridDim.x)) return;
         pAp = d[0];
       }
       alpha = (pAp == 0.0) ? 0.0 : rz / pAp;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(PR_THREADS, 1)
             d[1] += (double)r * (double)r;
           }
         }
-        if (!pr_barrier<2>(s, a, d, a.partials + gridDim.x)) return;
+        if (!pr_barrier<2>(s, a, d, a.partials + PCG_SUM_B * gridDim.x)) return;
         rz_new = d[0];
         rsq = d[1];
       }
