@@ -118,6 +118,7 @@ SIGNATURES = {
                                         _P, _P, _P]),
     "bsp_spmv": (_I, [_P, _P, _P, _I, _I, _I, _P]),
     "bsp_selftest_div6": (_I, [_P, _P]),
+    "bsp_selftest_div_by": (_I, [_P, _F, _P]),
     "bsp_selftest_waits": (_I, [_P, _P, _P]),
     "bsp_solve_params_default": (None, [_P]),
     "bsp_solver_workspace_bytes": (ctypes.c_size_t, [_I, _I, _I, _I]),

@@ -39,7 +39,7 @@ namespace sl {
 struct Geo {
   int nx, ny, nz;
   int planes;  // of a CTA, at most PL
-  float ox, oy, oz, dx, dt, rdx;  // rdx = 1 / dx, correctly rounded
+  float ox, oy, oz, dx, dt, rdx, least;  // rdx, least: for div_by
 };
 
 constexpr int BK = 32, BJ = 8, PL = 8;  // CTA: 32 k x 8 j, marching up to 8 planes
@@ -162,9 +162,9 @@ __device__ __forceinline__ float advected(const float *__restrict__ f, const Coo
   const float qx = __fsub_rn(c.px[LX][ii], __fmul_rn(u, g.dt));
   const float qy = __fsub_rn(c.py[LY][ty], __fmul_rn(v, g.dt));
   const float qz = __fsub_rn(c.pz[LZ][tx], __fmul_rn(w, g.dt));
-  const float bx = div_by(__fsub_rn(qx, g.ox), g.dx, g.rdx);
-  const float by = div_by(__fsub_rn(qy, g.oy), g.dx, g.rdx);
-  const float bz = div_by(__fsub_rn(qz, g.oz), g.dx, g.rdx);
+  const float bx = div_by(__fsub_rn(qx, g.ox), g.dx, g.rdx, g.least);
+  const float by = div_by(__fsub_rn(qy, g.oy), g.dx, g.rdx, g.least);
+  const float bz = div_by(__fsub_rn(qz, g.oz), g.dx, g.rdx, g.least);
   return tri(f, g.nx + !LX, g.ny + !LY, g.nz + !LZ, bx, by, bz, LX ? 0.5f : 0.0f,
              LY ? 0.5f : 0.0f, LZ ? 0.5f : 0.0f);
 }
@@ -408,7 +408,7 @@ extern "C" int bsp_extend_temperature(float *T_ext, const float *T, const uint8_
   if (!T_ext || !T || !mask) return BSP_ERR_NULL;
   if (T_ext == T) return BSP_ERR_ALIAS;
   if (!dims_ok(nx, ny, nz)) return BSP_ERR_SHAPE;
-  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 1.0f};
+  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 1.0f, 1.0f};
   return (int)launch_extend(T_ext, T, mask, g, s);
 }
 
@@ -420,7 +420,8 @@ extern "C" int bsp_advect_temperature(float *T_new, const float *T_true, const f
   if (!T_new || !T_true || !T_ext || !ux || !uy || !uz || !mask) return BSP_ERR_NULL;
   if (T_new == T_true || T_new == T_ext) return BSP_ERR_ALIAS;
   if (!dims_ok(nx, ny, nz) || !(dx > 0.0f)) return BSP_ERR_SHAPE;
-  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, 1.0f / dx};
+  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, bsp::rcp_of(dx),
+              bsp::div_least(bsp::rcp_of(dx))};
   advect_T_kernel<<<grid_pl(nx, ny, nz, g.planes), dim3(BK, BJ), 0, s>>>(T_new, T_true, T_ext, ux,
                                                                          uy, uz, mask, g);
   return (int)cudaGetLastError();
@@ -435,7 +436,8 @@ extern "C" int bsp_advect_velocity(int axis, float *u_new, const float *ux, cons
   if (axis < 0 || axis > 2) return BSP_ERR_ARG;
   if (u_new == ux || u_new == uy || u_new == uz) return BSP_ERR_ALIAS;
   if (!dims_ok(nx, ny, nz) || !(dx > 0.0f)) return BSP_ERR_SHAPE;
-  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, 1.0f / dx};
+  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, bsp::rcp_of(dx),
+              bsp::div_least(bsp::rcp_of(dx))};
   return (int)launch_velocity(axis, u_new, ux, uy, uz, mask, g, s);
 }
 
@@ -459,7 +461,8 @@ extern "C" int bsp_advect_all(float *ux, float *uy, float *uz, float *T, float *
       if (outs[a] == outs[b]) return BSP_ERR_ALIAS;
   }
   if (!dims_ok(nx, ny, nz) || !(dx > 0.0f)) return BSP_ERR_SHAPE;
-  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, 1.0f / dx};
+  const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, bsp::rcp_of(dx),
+              bsp::div_least(bsp::rcp_of(dx))};
   cudaError_t e = cudaSuccess;
   e = launch_extend(T_ext, T, mask, g, s);
   if (e != cudaSuccess) return (int)e;

@@ -163,13 +163,25 @@ inline bool smem_opt_in(const void *fn, int bytes) {
   return ok;
 }
 
-// a / d, correctly rounded, with y = 1 / d correctly rounded: after one step the
+// 1 / d for div_by: correctly rounded, or 0 (then it divides) where that is near the end of
+// the normal range.
+__host__ __device__ __forceinline__ float rcp_of(float d) {
+  const float y = 1.0f / d;
+  return fabsf(y) > 1e-30f ? y : 0.0f;
+}
+// Least quotient for which div_by does not divide: |a| is then above 1e-30 too.
+constexpr float DIV_LEAST = 2e-30f;  // |d| >= 1
+__host__ __device__ __forceinline__ float div_least(float y) {
+  return DIV_LEAST * fmaxf(1.0f, fabsf(y));
+}
+// a / d, correctly rounded, with y = rcp_of(d) and least = div_least(y): after one step the
 // quotient is within a unit in the last place, and a step from there rounds as a
-// division does (Markstein) -- as long as nothing leaves the normal range, else
-// the division itself.
-__device__ __forceinline__ float div_by(float a, float d, float y) {
+// division does (Markstein) -- as long as the remainder a - q d is exact and nothing
+// leaves the normal range, else the division itself.  The remainder's last place is at least
+// 2^-48 |a|, a float's while |a| > 1e-30.  Checked over all a by bsp_selftest_div_by.
+__device__ __forceinline__ float div_by(float a, float d, float y, float least = DIV_LEAST) {
   float q = __fmul_rn(a, y);
-  if (!(fabsf(q) > 1e-30f && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
+  if (!(fabsf(q) > least && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
   q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
   return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
 }

@@ -401,8 +401,10 @@ __device__ __forceinline__ void build_class_table(float4 *tab, float *gt,
         diag = __fadd_rn(diag, g[f]);
       }
     }
-    tab[2 * c] = make_float4(__fadd_rn(1.0f, diag), g[0], g[1], g[2]);
-    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], __fdiv_rn(1.0f, __fadd_rn(1.0f, diag)));
+    const float den = __fadd_rn(1.0f, diag);
+    tab[2 * c] = make_float4(den, g[0], g[1], g[2]);
+    // for div_by (which divides where this is 0; below 1 only with a negative gamma)
+    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], den >= 1.0f ? rcp_of(den) : 0.0f);
   }
   __syncthreads();
 }

@@ -1,4 +1,5 @@
-// selftest.cu -- self-checks of the bounded device waits.
+// selftest.cu -- self-checks of the bounded device waits and of the division by a
+// reciprocal (bsp_common.cuh).
 //
 // Every spin in this library is bounded: the grid barrier of the persistent
 // kernels (grid_sync.cuh) gives up after BAR_TIMEOUT_NS on the global timer
@@ -28,7 +29,27 @@ __global__ void selftest_mbar_kernel(int *code) {
   if (threadIdx.x == 0) code[1] = mbar_wait(&bar, 0) ? BSP_OK : BSP_ERR_TIMEOUT;
 }
 
+// div_by against the division, over all 2^32 dividends (a NaN equals a NaN).
+__global__ void selftest_div_by_kernel(unsigned long long *bad, float d) {
+  const float y = rcp_of(d), least = div_least(y);
+  unsigned int n = 0;
+  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < (1ull << 32);
+       u += (uint64_t)gridDim.x * blockDim.x) {
+    const float a = __uint_as_float((uint32_t)u), q = div_by(a, d, y, least), w = __fdiv_rn(a, d);
+    if (__float_as_uint(q) != __float_as_uint(w) && !(isnan(q) && isnan(w))) ++n;
+  }
+  if (n) atomicAdd(bad, (unsigned long long)n);
+}
+
 }  // namespace bsp
+
+extern "C" int bsp_selftest_div_by(unsigned long long *mismatches_dev, float d, cudaStream_t s) {
+  if (!mismatches_dev) return BSP_ERR_NULL;
+  cudaError_t e = cudaMemsetAsync(mismatches_dev, 0, sizeof(unsigned long long), s);
+  if (e != cudaSuccess) return (int)e;
+  bsp::selftest_div_by_kernel<<<148 * 8, 256, 0, s>>>(mismatches_dev, d);
+  return (int)cudaGetLastError();
+}
 
 extern "C" int bsp_selftest_waits(int *codes_dev, void *scratch_dev, cudaStream_t s) {
   using namespace bsp;

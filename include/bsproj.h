@@ -661,6 +661,10 @@ int bsp_unet_energy_scale_keep(float *p, const float *Ap, const float *div, cons
  * device counter *mismatches_dev (zeroed first). */
 int bsp_selftest_div6(unsigned long long *mismatches_dev, cudaStream_t stream);
 
+/* The number of dividends, of all 2^32, on which the division by a precomputed
+ * reciprocal (conduction, advection, PCG) differs from IEEE division by d. */
+int bsp_selftest_div_by(unsigned long long *mismatches_dev, float d, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
