@@ -185,5 +185,12 @@ __device__ __forceinline__ float div_by(float a, float d, float y, float least =
   q = __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
   return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
 }
+// The same for d = 1 .. 6, y = 1 / d correctly rounded: the product is within a place of the
+// quotient, so one step is enough (checked over all a by the same self-test).
+__device__ __forceinline__ float div_small(float a, float d, float y) {
+  const float q = __fmul_rn(a, y);
+  if (!(fabsf(q) > DIV_LEAST && fabsf(q) < 1e30f)) return __fdiv_rn(a, d);
+  return __fmaf_rn(__fmaf_rn(-d, q, a), y, q);
+}
 
 }  // namespace bsp

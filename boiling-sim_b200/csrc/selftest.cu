@@ -29,14 +29,18 @@ __global__ void selftest_mbar_kernel(int *code) {
   if (threadIdx.x == 0) code[1] = mbar_wait(&bar, 0) ? BSP_OK : BSP_ERR_TIMEOUT;
 }
 
-// div_by against the division, over all 2^32 dividends (a NaN equals a NaN).
+// div_by, and div_small for its divisors, against the division, over all 2^32 dividends (a
+// NaN equals a NaN).
 __global__ void selftest_div_by_kernel(unsigned long long *bad, float d) {
   const float y = rcp_of(d), least = div_least(y);
+  const bool small = d == 1.0f || d == 2.0f || d == 3.0f || d == 4.0f || d == 5.0f || d == 6.0f;
   unsigned int n = 0;
   for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < (1ull << 32);
        u += (uint64_t)gridDim.x * blockDim.x) {
     const float a = __uint_as_float((uint32_t)u), q = div_by(a, d, y, least), w = __fdiv_rn(a, d);
     if (__float_as_uint(q) != __float_as_uint(w) && !(isnan(q) && isnan(w))) ++n;
+    const float v = small ? div_small(a, d, y) : w;
+    if (__float_as_uint(v) != __float_as_uint(w) && !(isnan(v) && isnan(w))) ++n;
   }
   if (n) atomicAdd(bad, (unsigned long long)n);
 }
