@@ -1,9 +1,10 @@
 // autotune.cu -- the library's autotuner: times the candidate tile shapes and
 // pass depths of a kernel family on the caller's own problem and keeps the
-// fastest (bsp_set_tuning), so later calls of the same family use it.
+// fastest, so later calls of the same family use it.
 //
 //   bsp_autotune_jacobi: sweep plane chunk (BSP_TUNE_SWEEP_BI) x sweeps per
-//     HBM pass (BSP_TUNE_SWEEP_TBLOCK: one, or two temporally blocked);
+//     HBM pass (BSP_TUNE_SWEEP_TBLOCK: by size, one, or two temporally blocked),
+//     kept for grids of that size;
 //   bsp_autotune_solve: plane chunk of the solver's level-0 tiles
 //     (BSP_TUNE_FINE_BI) x the one-launch coarse cycle (BSP_TUNE_COARSE_FUSED).
 //
@@ -16,9 +17,12 @@
 #include <vector>
 
 #include "../../include/bsproj.h"
+#include "bsp_common.cuh"
 
 namespace bsp {
 extern int g_sweep_bi, g_sweep_tblock, g_fine_bi;
+extern SweepTune g_sweep_tuned[3];
+int sweep_size(int64_t n);
 extern bool g_coarse_fused_enabled;
 int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                       const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
@@ -27,6 +31,8 @@ int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
 }  // namespace bsp
 
 namespace {
+
+__device__ unsigned int g_tune_bar;  // barrier word of the one-launch sweeps while they are timed
 
 struct Timer {
   cudaEvent_t a = nullptr, b = nullptr;
@@ -54,25 +60,36 @@ extern "C" int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, f
   using namespace bsp;
   if (!p || !p_tmp || !div_u || !rhs_ws || !mask || !n_out) return BSP_ERR_NULL;
   if (nx <= 0 || ny <= 0 || nz <= 0 || sweeps < 2) return BSP_ERR_ARG;
+  // plane chunks x single or paired sweeps; the first candidate is the default, which
+  // chooses by size and runs small grids in one launch
   const int bis[] = {0, 2, 4, 8, 16, 32};
   const int depths[] = {1, 2};
   const int save_bi = g_sweep_bi, save_tb = g_sweep_tblock;
+  const int64_t n = (int64_t)nx * ny * nz;
+  SweepTune &tuned = g_sweep_tuned[sweep_size(n)];
+  const SweepTune saved = tuned;
+  SweepTune choice = saved;
+  unsigned int *bar = nullptr;  // barrier word of the one-launch form
+  cudaError_t be = cudaGetSymbolAddress((void **)&bar, g_tune_bar);
+  if (be != cudaSuccess) return (int)be;
   Timer t;
   float best = 1e30f;
-  int best_bi = save_bi, best_tb = save_tb;
   *n_out = 0;
-  const size_t bytes = sizeof(float) * (size_t)nx * ny * nz;
-  for (int tb : depths)
+  const size_t bytes = sizeof(float) * (size_t)n;
+  g_sweep_tblock = 0;
+  tuned = SweepTune{};
+  for (int depth : depths)
     for (int bi : bis) {
+      const int tb = depth == 1 && bi == 0 ? 0 : depth;
       g_sweep_bi = bi;
-      g_sweep_tblock = tb;
       int st = BSP_OK;
       float ms = 0.0f;
       for (int rep = 0; rep < 2 && st == BSP_OK; ++rep) {  // untimed, then timed
         cudaMemsetAsync(p, 0, bytes, s);
+        cudaMemsetAsync(p_tmp, 0, bytes, s);
         cudaEventRecord(t.a, s);
         st = jacobi_solve_impl(p, p_tmp, div_u, rhs_ws, mask, nx, ny, nz, dx, dt, rho, sweeps,
-                               0, s, true, false, nullptr);
+                               tb, s, true, true, bar);
         cudaEventRecord(t.b, s);
       }
       if (st == BSP_OK) st = (int)cudaEventSynchronize(t.b);
@@ -81,12 +98,14 @@ extern "C" int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, f
       put(out, max_out, n_out, BSP_TUNE_SWEEP_BI, bi | (tb << 16), per, st);
       if (st == BSP_OK && per < best) {
         best = per;
-        best_bi = bi;
-        best_tb = tb;
+        choice.bi = bi;
+        choice.tblock = tb;
       }
     }
-  g_sweep_bi = best_bi;
-  g_sweep_tblock = best_tb;
+  const bool found = best < 1e30f;  // then it takes the place of what the keys said
+  g_sweep_bi = found ? 0 : save_bi;
+  g_sweep_tblock = found ? 0 : save_tb;
+  tuned = choice;
   return (int)cudaGetLastError();
 }
 

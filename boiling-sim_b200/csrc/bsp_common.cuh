@@ -163,6 +163,14 @@ inline bool smem_opt_in(const void *fn, int bytes) {
   return ok;
 }
 
+// Jacobi sweeps as tuned for grids of a size (0: at most ONCHIP_SWEEP_CELLS cells, 1: in L2, 2:
+// larger; sweep_size): plane chunk of the march (0: the rule), and sweeps per pass as in
+// BSP_TUNE_SWEEP_TBLOCK, but 1 here means single sweeps also where all would fit in one launch.
+struct SweepTune {
+  int bi = 0, tblock = 0;
+};
+constexpr int64_t ONCHIP_SWEEP_CELLS = 2LL << 20;
+
 // 1 / d for div_by: correctly rounded, or 0 (then it divides) where that is near the end of
 // the normal range.
 __host__ __device__ __forceinline__ float rcp_of(float d) {

@@ -27,13 +27,15 @@ cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const
 // which leaves +0 there, so from the second sweep on the ZNF kernel applies.
 bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *mask, int nx,
                    int ny, int nz, cudaStream_t s);
-// BSP_TUNE_SWEEP_TBLOCK: sweeps per pass when a call passes 0 (0: the rule below)
+// BSP_TUNE_SWEEP_TBLOCK: sweeps per pass when a call passes 0 (0 and 1: the rule below)
 int g_sweep_tblock = 0;
+extern SweepTune g_sweep_tuned[3];
+int sweep_size(int64_t n);
 // sweepr.cu: all sweeps in one launch; false when the grid does not fit
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
                      int nz, int n, unsigned int *bar, cudaStream_t s, cudaError_t *e);
 
-// n_iter sweeps p <-> p_tmp, result in p.  tblock 0 (and no autotuned depth): the
+// n_iter sweeps p <-> p_tmp, result in p.  tblock 0 (and no depth tuned for this size): the
 // whole solve in one launch with the pressure resident in shared memory where
 // that fits (p and p_tmp start at zero, the right-hand side hoisted, and bar, 4
 // bytes of device memory for a grid barrier, given), else one sweep per
@@ -52,7 +54,8 @@ int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
     cudaError_t e = launch_rhs(rhs_ws, div_u, mask, n, dx, dt, rho, stream);
     if (e != cudaSuccess) return (int)e;
   }
-  const int depth = tblock > 0 ? tblock : g_sweep_tblock;
+  const int depth =
+      tblock > 0 ? tblock : (g_sweep_tblock > 1 ? g_sweep_tblock : g_sweep_tuned[sweep_size(n)].tblock);
   if (depth == 0 && rhs_ws && p_zero && tmp_zero) {
     cudaError_t e = cudaSuccess;
     if (sweeps_resident(p, p_tmp, rhs_ws, mask, nx, ny, nz, n_iter, bar, stream, &e)) return (int)e;

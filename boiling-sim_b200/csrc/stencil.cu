@@ -499,6 +499,10 @@ __global__ void __launch_bounds__(256, VEC == 4 ? 5 : 6)
 int g_sweep_prefetch = 2;
 // Cells up to which a sweep's fields (13 B a cell) count as resident in L2.
 constexpr int64_t L2_SWEEP_CELLS = 10LL << 20;
+// What bsp_autotune_jacobi has chosen (bsp_common.cuh), by the size of its grid: the three
+// sizes are swept by kernels of their own, and what is best for one says nothing of the others.
+SweepTune g_sweep_tuned[3];
+int sweep_size(int64_t n) { return n <= ONCHIP_SWEEP_CELLS ? 0 : (n <= L2_SWEEP_CELLS ? 1 : 2); }
 
 // ---- generic kernel -----------------------------------------------------------
 template <int OP, class MaskT>
@@ -631,6 +635,10 @@ static inline int generic_blocks(int64_t n) {
 // while keeping the i-halo re-read (2/bi) small.
 // Autotuner override of the column kernel's i-extent (0 = heuristic below).
 int g_sweep_bi = 0;
+// the plane chunk that was set for grids of n cells (0: none)
+int sweep_bi_set(int64_t n) {
+  return g_sweep_bi > 0 ? g_sweep_bi : g_sweep_tuned[sweep_size(n)].bi;
+}
 
 static inline int pick_bi(int nx, int ny, int nz) {
   const int64_t cols = (int64_t)((nz / 4 + 31) / 32) * ((ny + 7) / 8);
@@ -649,7 +657,7 @@ cudaError_t launch_stencil(float *out, const float *p, const float *div, const M
                       (OP == OP_SPMV || aligned16(div)) &&
                       (sizeof(MaskT) == 4 ? aligned16(mask) : (((uintptr_t)mask & 3u) == 0));
   if (col_ok) {
-    const int bi = g_sweep_bi > 0 ? g_sweep_bi : pick_bi(nx, ny, nz);
+    const int set = sweep_bi_set((int64_t)nx * ny * nz), bi = set > 0 ? set : pick_bi(nx, ny, nz);
     dim3 grid((nz / 4 + 31) / 32, (ny + 7) / 8, (nx + bi - 1) / bi);
     if (nz % 128 == 0)
       stencil_col_kernel<OP, MaskT, true><<<grid, 256, 0, s>>>(out, p, div, mask, nx, ny, nz, bi,
@@ -678,16 +686,16 @@ cudaError_t launch_point(float *out, const float *p, const float *rhs, const uin
 // off fluid already.  pdl: the kernel before in the stream is a sweep of the
 // same solve.  Bit-identical to launch_stencil<OP_JACOBI_RHS>.
 // The march (aligned rows only) serves the grids whose fields (13 B a cell) do
-// not stay in L2, and a plane chunk set by the autotuner; the point kernel the
-// rest.  Measured on pots, us a sweep, march / point: 192x192x128 13.4 / 9.9,
+// not stay in L2, and a plane chunk that was set, by the tuning key or by the autotuner for
+// grids of this size; the point kernel the rest.  Measured on pots, us a sweep, march / point: 192x192x128 13.4 / 9.9,
 // 384x384x256 76 / 82.
 cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const uint8_t *mask,
                              int nx, int ny, int nz, bool fill, bool pdl, cudaStream_t s) {
   const bool vec = (nz % 4 == 0) && aligned16(out) && aligned16(p) && aligned16(rhs) &&
                    (((uintptr_t)mask & 3u) == 0);
   const int64_t n = (int64_t)nx * ny * nz;
-  if (nx <= 65535 && (ny + 7) / 8 <= 65535 &&
-      (!vec || (n <= L2_SWEEP_CELLS && g_sweep_bi == 0))) {
+  const int set = sweep_bi_set(n);
+  if (nx <= 65535 && (ny + 7) / 8 <= 65535 && (!vec || (n <= L2_SWEEP_CELLS && set == 0))) {
     auto fn = vec ? (fill ? launch_point<4, true> : launch_point<4, false>)
                   : (fill ? launch_point<1, true> : launch_point<1, false>);
     return fn(out, p, rhs, mask, nx, ny, nz, pdl, s);
@@ -695,7 +703,7 @@ cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const
   if (!vec)
     return launch_stencil<OP_JACOBI_RHS, uint8_t>(out, p, rhs, mask, nx, ny, nz, 0.f, 1.f, 0.f,
                                                   BSP_FLUID, BSP_AIR, s);
-  const int bi = g_sweep_bi > 0 ? g_sweep_bi : pick_bi(nx, ny, nz);
+  const int bi = set > 0 ? set : pick_bi(nx, ny, nz);
   dim3 grid((nz / 4 + 31) / 32, (ny + 7) / 8, (nx + bi - 1) / bi);
   if (nz % 128 == 0)
     (g_sweep_prefetch == 3   ? sweep_znf_kernel<true, 3>
@@ -880,6 +888,7 @@ extern "C" int bsp_set_tuning(int key, int value) {
     case BSP_TUNE_SWEEP_BI:
       if (value < 0 || value > 4096) return BSP_ERR_ARG;
       bsp::g_sweep_bi = value;
+      for (bsp::SweepTune &t : bsp::g_sweep_tuned) t.bi = 0;
       return BSP_OK;
     case BSP_TUNE_FINE_COLUMN:
       if (value < 0 || value > 1) return BSP_ERR_ARG;
@@ -906,8 +915,9 @@ extern "C" int bsp_set_tuning(int key, int value) {
       bsp::g_fine_bi = value;
       return BSP_OK;
     case BSP_TUNE_SWEEP_TBLOCK:
-      if (value < 1 || value > 2) return BSP_ERR_ARG;
+      if (value < 0 || value > 2) return BSP_ERR_ARG;
       bsp::g_sweep_tblock = value;
+      for (bsp::SweepTune &t : bsp::g_sweep_tuned) t.tblock = 0;
       return BSP_OK;
     case BSP_TUNE_COND_BI:
       if (value < 0 || value > 4096) return BSP_ERR_ARG;
@@ -992,6 +1002,26 @@ extern "C" int bsp_set_tuning(int key, int value) {
     case BSP_TUNE_TEST_BARRIER_ERROR:
       if (value < 0 || value > 1) return BSP_ERR_ARG;
       bsp::g_test_barrier_error = value != 0;
+      return BSP_OK;
+    default:
+      return BSP_ERR_ARG;
+  }
+}
+
+extern "C" int bsp_get_tuning(int key, int *value) {
+  if (!value) return BSP_ERR_NULL;
+  switch (key) {
+    case BSP_TUNE_SWEEP_BI:
+      *value = bsp::g_sweep_bi;
+      return BSP_OK;
+    case BSP_TUNE_SWEEP_TBLOCK:
+      *value = bsp::g_sweep_tblock;
+      return BSP_OK;
+    case BSP_TUNE_FINE_BI:
+      *value = bsp::g_fine_bi;
+      return BSP_OK;
+    case BSP_TUNE_COARSE_FUSED:
+      *value = bsp::g_coarse_fused_enabled;
       return BSP_OK;
     default:
       return BSP_ERR_ARG;

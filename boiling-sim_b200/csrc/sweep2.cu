@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(sw2::THREADS, 2) sweep2_kernel(
 // launch are then not valid); read back by bsp_sweep2_error.
 __device__ int g_sweep2_err;
 int num_sms();
-extern int g_sweep_bi;  // BSP_TUNE_SWEEP_BI (stencil.cu)
+int sweep_bi_set(int64_t n);  // plane chunk set for grids of n cells, or 0 (stencil.cu)
 
 int *sweep2_error_word() {
   int *err = nullptr;
@@ -245,7 +245,7 @@ bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *
   const int64_t cols = (int64_t)((nz + 127) / 128) * ((ny + ROWS - 1) / ROWS);
   int bi = 16;
   while (bi > 2 && cols * ((nx + bi - 1) / bi) < 2LL * num_sms()) bi -= 2;
-  if (g_sweep_bi > 0) bi = g_sweep_bi;
+  if (const int set = sweep_bi_set((int64_t)nx * ny * nz)) bi = set;
   dim3 grid((nz + 127) / 128, (ny + ROWS - 1) / ROWS, (nx + bi - 1) / bi);
   sweep2_kernel<<<grid, THREADS, TOTAL, s>>>(out, maps, nx, ny, nz, bi, err);
   return cudaGetLastError() == cudaSuccess;

@@ -59,7 +59,8 @@ extern "C" {
 #define BSP_TUNE_COARSE_FUSED 5 /* coarse V-cycle levels in one cooperative kernel: 1 on, 0 off */
 #define BSP_TUNE_FUSE_UPDATE 6  /* CG update fused into the next restriction (TMA path): 1 on, 0 off */
 #define BSP_TUNE_FINE_BI 7      /* i-planes per CTA tile of the solver's level-0 kernels (0 = rule) */
-#define BSP_TUNE_SWEEP_TBLOCK 8 /* sweeps per HBM pass when a call passes tblock = 0 (1, 2; 0: by size) */
+#define BSP_TUNE_SWEEP_TBLOCK 8 /* sweeps per HBM pass when a call passes tblock = 0: 0 (default), 1: one, or
+                                   all in one launch where they fit on chip; 2: two */
 #define BSP_TUNE_COND_BI 9      /* i-planes per CTA of the conduction sweeps (0 = rule) */
 #define BSP_TUNE_COND_TMA 10    /* conduction class sweep fed by TMA tiles: 1 on, 0 off */
 /* Tests only: 1 makes the next host-driven bsp_solve_tol start with the
@@ -213,6 +214,9 @@ int bsp_sweep2_error(int *flag_host);
 /* Set an autotuner parameter (BSP_TUNE_*) for subsequent launches in this
  * process.  Not thread-safe against concurrent launches. */
 int bsp_set_tuning(int key, int value);
+/* The value of BSP_TUNE_SWEEP_BI, BSP_TUNE_SWEEP_TBLOCK, BSP_TUNE_FINE_BI or
+ * BSP_TUNE_COARSE_FUSED. */
+int bsp_get_tuning(int key, int *value);
 
 /* Per-kernel-class event timing (tracing).  While enabled, every launch of an
  * instrumented kernel is bracketed by CUDA events on its stream.  Classes:
@@ -376,9 +380,9 @@ int bsp_solve_batch(int count, const BspBatchItem *items, const BspSolveParams *
 /* ---- autotuner ------------------------------------------------------------
  * Time the candidate decompositions of a kernel family on the caller's own
  * problem (CUDA events on `stream`, one untimed run first) and keep the
- * fastest through bsp_set_tuning.  out[0 .. min(*n_out, max_out)) receives
+ * fastest.  out[0 .. min(*n_out, max_out)) receives
  * one row per candidate: key, value (low 16 bits: the plane chunk, 0 = rule;
- * bit 16: the second switch), milliseconds (per sweep / per solve) and the
+ * from bit 16: the second switch), milliseconds (per sweep / per solve) and the
  * candidate's status.  The buffers are overwritten.  No reference
  * counterpart (the reference has no tuning step). */
 typedef struct BspTuneChoice {
@@ -387,8 +391,11 @@ typedef struct BspTuneChoice {
   int status;
 } BspTuneChoice;
 
-/* Sweep plane chunk x sweeps per HBM pass (one, or two temporally blocked);
- * `sweeps` sweeps per candidate on p / p_tmp / rhs_ws (p is zeroed first). */
+/* Sweep plane chunk x sweeps per HBM pass (bit 16 on: 0 the default, which runs
+ * small grids in one launch; one; or two temporally blocked); `sweeps` sweeps
+ * per candidate on p / p_tmp / rhs_ws (p and p_tmp are zeroed first).  The choice
+ * holds for grids of this size (up to 2 M cells, up to 10 M, larger), until
+ * BSP_TUNE_SWEEP_BI or BSP_TUNE_SWEEP_TBLOCK is set. */
 int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                         const uint8_t *mask, int nx, int ny, int nz, float dx, float dt,
                         float rho, int sweeps, BspTuneChoice *out, int max_out, int *n_out,
