@@ -24,6 +24,7 @@ extern int g_sweep_bi, g_sweep_tblock, g_fine_bi;
 extern SweepTune g_sweep_tuned[3];
 int sweep_size(int64_t n);
 extern bool g_coarse_fused_enabled;
+bool group_eligible(int nx, int ny, int nz);
 int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                       const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
                       int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero,
@@ -152,7 +153,10 @@ extern "C" int bsp_autotune_solve(float *p, const float *div_u, const uint8_t *m
         best_fused = fz;
       }
     }
-  g_fine_bi = best_bi;
-  g_coarse_fused_enabled = best_fused;
+  // a grid of the one-launch solve has no tiles: its times differ by noise alone, and the
+  // settings are those of the grids that have
+  const bool tiles = !group_eligible(nx, ny, nz);
+  g_fine_bi = tiles ? best_bi : save_bi;
+  g_coarse_fused_enabled = tiles ? best_fused : save_fused;
   return (int)cudaGetLastError();
 }

@@ -929,7 +929,7 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
 // per-kernel path also serves what the group kernel has not: per-kernel tracing,
 // trilinear transfers, the barrier-error test.
 constexpr int64_t GROUP_CELLS = 24LL << 20;
-static bool group_eligible(int nx, int ny, int nz) {
+bool group_eligible(int nx, int ny, int nz) {
   if (!g_group_solve || g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
   if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
   const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);

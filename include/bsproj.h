@@ -402,7 +402,9 @@ int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, float *rhs_w
                         cudaStream_t stream);
 
 /* Plane chunk of the to-tolerance solver's level-0 tiles x the one-launch
- * coarse cycle, each candidate a full bsp_solve_tol with `params`. */
+ * coarse cycle, each candidate a full bsp_solve_tol with `params`.  On a grid
+ * that is solved in one launch the candidates do not differ, and both settings
+ * stay as they are. */
 int bsp_autotune_solve(float *p, const float *div_u, const uint8_t *mask, int nx, int ny,
                        int nz, float dx, float dt, float rho, const struct BspSolveParams *params,
                        void *workspace, size_t workspace_bytes, BspTuneChoice *out, int max_out,
