@@ -87,14 +87,14 @@ def test_default_can_be_set(cuda):
 
 
 def test_autotuner_times_the_one_launch_form(cuda):
-    """Twice, as the first candidate; the others sweep one at a time (rows of 38 cells have no
-    pairs).  The fastest is used afterwards."""
-    rows, launches = _sweep_launches(lambda: _tune((58, 58, 38)))
+    """Twice, as the first candidate; the others sweep one by one or in pairs.  The fastest is
+    used afterwards."""
+    rows, launches = _sweep_launches(lambda: _tune((58, 58, 48)))
     assert len(rows) == 12 and all(r["status"] == 0 for r in rows)
     assert (rows[0]["plane_chunk"], rows[0]["sweeps_per_pass"]) == (0, 0)
-    assert launches == 2 + 11 * 2 * 20
-    first = rows[0]["ms_per_sweep"] == min(r["ms_per_sweep"] for r in rows)
-    assert _project(*_scene((58, 58, 38)), 9)[1] == (1 if first else 9)
+    assert launches == 2 + 5 * 2 * 20 + 6 * 2 * 10
+    best = min(rows, key=lambda r: r["ms_per_sweep"])["sweeps_per_pass"]
+    assert _project(*_scene((58, 58, 48)), 9)[1] == {0: 1, 1: 9, 2: 5}[best]
 
 
 def test_tuning_a_large_grid_leaves_the_small_ones_alone(cuda):
