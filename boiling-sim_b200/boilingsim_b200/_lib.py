@@ -42,6 +42,7 @@ SIGNATURES = {
     "bsp_jacobi_solve": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _F, _F, _F, _I, _I, _P]),
     "bsp_set_tuning": (_I, [_I, _I]),
     "bsp_get_tuning": (_I, [_I, _P]),
+    "bsp_wait_status": (_I, [_I]),
     "bsp_sweep2_error": (_I, [_P]),
     "bsp_autotune_jacobi": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _F, _F, _F, _I, _P, _I, _P, _P]),
     "bsp_autotune_solve": (_I, [_P, _P, _P, _I, _I, _I, _F, _F, _F, _P, _P, ctypes.c_size_t, _P,

@@ -30,6 +30,7 @@ from . import _lib
 from ._lib import call, ptr, stream_handle
 
 MAT_FLUID, MAT_POT_WALL, MAT_AIR, MAT_CARROT = 0, 1, 2, 3
+WAIT_SWEEPS = 0  # bsp_wait_status
 
 
 @dataclass
@@ -245,7 +246,15 @@ def pressure_projection(grid: Grid, ws: FluidWorkspace, cfg: ScenarioConfig, dt:
         torch.cuda.synchronize()
         subtract_pressure_gradient(grid.ux, grid.uy, grid.uz, grid.p, mask, dx, dt, rho)
         compute_divergence(ws.div_u, grid.ux, grid.uy, grid.uz, mask, dx, ws.max_div)
-    return float(ws.max_div.item())
+    return _waited(ws.max_div)
+
+
+def _waited(max_div: torch.Tensor) -> float:
+    """The diagnostic, once its stream has been waited for; raises if the sweeps gave up a
+    bounded device-side wait (the pressure and velocities are then not valid)."""
+    out = float(max_div.item())
+    call("bsp_wait_status", WAIT_SWEEPS)
+    return out
 
 
 _STORAGE = {"b200-mg": "fp32", "b200-mixed": "fp16", "b200-bf16": "bf16",
@@ -370,7 +379,7 @@ class ProjectionPipeline:
         if slot.get("ticket") != ticket:
             raise ValueError("that projection's slot has been reused; take results in order")
         slot["done"].synchronize()
-        return float(slot["max_div"].item())
+        return _waited(slot["max_div"])
 
 
 _NET = None
@@ -446,7 +455,7 @@ def projection_step(grid: Grid, ws: FluidWorkspace, cfg: ScenarioConfig, dt: flo
         call("bsp_step_projection_jacobi", ptr(grid.p), ptr(ws.p_tmp), ptr(ws.div_u),
              ptr(grid.ux), ptr(grid.uy), ptr(grid.uz), ptr(mask), nx, ny, nz, dx, float(dt),
              float(rho), int(cfg.solver.pressure_max_iter), 0, ptr(ws.max_div), stream_handle())
-        return float(ws.max_div.item())
+        return _waited(ws.max_div)
     if solver.startswith("b200-"):
         noslip_divergence(ws.div_u, grid.ux, grid.uy, grid.uz, mask, dx)
         _tol_projection(grid, ws, cfg, solver, dt, rho)

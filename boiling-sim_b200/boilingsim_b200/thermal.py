@@ -202,7 +202,11 @@ def apply_implicit_conduction_update(T_dst, T_iter, T_old, mat, k_arr, rho_arr, 
 
 def implicit_conduction_step(grid, props: MaterialProps, ws: ThermalWorkspace, cfg, dt: float,
                              device: str = "cuda:0", stream=None) -> None:
-    """The backward-Euler branch of ``conduct_one_step`` (thermal.py:647-658)."""
+    """The backward-Euler branch of ``conduct_one_step`` (thermal.py:647-658).
+
+    Only enqueues the step.  If an earlier one gave up a bounded device-side wait (its
+    temperatures are then not valid), this raises ``BspError`` with code 10007 instead;
+    ``bsp_wait_status(1)`` asks the same after a synchronisation."""
     del device
     _check_f32(grid.T, ws.T_iter_alt, ws.T_old_snapshot)
     nx, ny, nz = grid.shape

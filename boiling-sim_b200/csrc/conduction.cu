@@ -42,8 +42,10 @@
 #include "bsp_common.cuh"
 #include "grid_sync.cuh"
 #include "tma.cuh"
+#include "waits.cuh"
 
 namespace bsp {
+extern int g_test_wait_error;  // BSP_TUNE_TEST_WAIT_ERROR (stencil.cu)
 int num_sms();
 
 namespace cond {
@@ -563,8 +565,6 @@ struct CondMaps {
   CUtensorMap t, c, o;
 };
 
-__device__ int g_cond_err;
-
 __device__ __forceinline__ float4 lds4(const float *p) {
   return *reinterpret_cast<const float4 *>(p);
 }
@@ -585,7 +585,7 @@ template <bool SNAP>
 __global__ void __launch_bounds__(tmac::THREADS + 32, 4) be_cls_tma_kernel(
     float *__restrict__ dst, float *__restrict__ snap, const __grid_constant__ CondMaps maps,
     const uint32_t *__restrict__ patterns, int ncls, const uint8_t *__restrict__ tiles, int nx,
-    int ny, int nz, int bi, Params P) {
+    int ny, int nz, int bi, Params P, int *err) {
   using namespace tmac;
   extern __shared__ __align__(128) unsigned char dsm[];
   __shared__ uint8_t s_own[MAX_BI + 4];  // tile occupancy of planes pbase-1 .. i1+1
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(tmac::THREADS + 32, 4) be_cls_tma_kernel(
         const uint32_t n = (uint32_t)(p - pbase);
         if (!mbar_wait(&full[n & (NST - 1)], (n / NST) & 1u)) ok = false;
       }
-      if (!ok) atomicExch(&g_cond_err, 1);
+      if (!ok) wait_gave_up(err);
     }
     return;
   }
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(tmac::THREADS + 32, 4) be_cls_tma_kernel(
     sc = sn;
   }
   // plane i1 (the last one read) is in stage sc: nothing refills it, no release needed
-  if (!ok) atomicExch(&g_cond_err, 1);
+  if (!ok) wait_gave_up(err);
 }
 
 // Tile occupancy for the TMA sweep: tiles[(i * TY + j / ROWS) * TX + k / 128]
@@ -892,7 +892,8 @@ struct Args {
   const void *mat;  // class bytes, or material ids
   const uint32_t *patterns;
   unsigned int *bar;  // arrivals, leavers
-  int *err;
+  int *err;           // marked when the barrier gave up
+  int extra;          // as in sweepr.cu
   int ncls, nx, ny, nz, nbx, nby, pad, cap, cols, n_iter;
   Params P;
 };
@@ -1018,30 +1019,24 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
   }
 
   unsigned int epoch = 0;
-  auto barrier = [&]() {  // arrivals on a counter that only grows; bounded
+  auto barrier = [&]() {
     __syncthreads();
-    if (tid == 0) {
-      const unsigned int target = ++epoch * gridDim.x;
-      cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(a.bar[0]);
-      cuda::atomic_ref<int, cuda::thread_scope_device> err(*a.err);
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      cnt.fetch_add(1u, cuda::memory_order_relaxed);
-      unsigned int spins = 0;
-      unsigned long long t0 = 0;
-      while (cnt.load(cuda::memory_order_acquire) < target) {
-        if ((++spins & 255u) == 0) {
-          const unsigned long long now = gs_global_ns();
-          if (t0 == 0) t0 = now;
-          if (now - t0 > BAR_TIMEOUT_NS || spins > BAR_SPIN_LIMIT) {
-            err.store(1, cuda::memory_order_relaxed);
-            s_ok = 0;
-            break;
-          }
-        }
-      }
+    if (tid == 0 && !counter_barrier(a.bar, ++epoch * gridDim.x + a.extra)) {
+      wait_gave_up(a.err);
+      s_ok = 0;
     }
     __syncthreads();
     return s_ok != 0;
+  };
+  // The last CTA to leave, after a barrier that gave up too, takes the barrier's words out of
+  // the snapshot: every CTA is past its last poll of them then.
+  auto leave = [&]() {
+    if (tid != 0) return;
+    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> left(a.bar[1]);
+    if (left.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
+      a.To[0] = t01[0];
+      a.To[1] = t01[1];
+    }
   };
 
   // ---- sweeps --------------------------------------------------------------------------
@@ -1085,7 +1080,7 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
       }
     }
     if (last) break;
-    if (!barrier()) return;
+    if (!barrier()) return leave();
     constexpr int HQ = 4;  // loads in flight
     for (int n0 = warp; n0 < halo; n0 += HQ * WARPS) {
       float v[HQ];
@@ -1111,7 +1106,7 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
   // ---- the last two iterates -----------------------------------------------------------
   // Odd: a CTA may still read the sides of iterate n - 1 in T.
   const bool odd = a.n_iter & 1;
-  if (odd && !barrier()) return;
+  if (odd && !barrier()) return leave();
   for (int t = tid; t < nc; t += THREADS) {
     const int at = (int)(E[t] & 0xffffu), c = gp[E[t] >> 24] + at;
     a.T[c] = nxt[at];
@@ -1123,14 +1118,7 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
       const int c = gp[col] + (li + 1) * di + (lj + 1) * dk + 1 + (l - col * nz);
       if (is_air(c)) a.T[c] = a.Ta[c];
     }
-  if (tid == 0) {
-    // every CTA is past its last poll of the words when the last one is here
-    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> left(a.bar[1]);
-    if (left.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
-      a.To[0] = t01[0];
-      a.To[1] = t01[1];
-    }
-  }
+  leave();
 }
 
 // True when the sweeps have been launched.  A block's cells all need a slot (what is air is
@@ -1148,10 +1136,15 @@ bool launch(float *T, float *Ta, float *To, const MatT *mat, const uint32_t *pat
   const int64_t cells = (int64_t)b.w * b.h * nz, halo = 2LL * (b.w + b.h) * ((nz + 31) / 32);
   const int64_t bytes = 4 * (2 * pad + (CLS ? 1 : 2) * cells + b.w * b.h + 1 + 3 * halo);
   if (b.w * b.h > COLS || pad > (1 << 16) || cells > SLOTS * THREADS || bytes > SMEM) return false;
-  int *err = nullptr;
-  if (cudaGetSymbolAddress((void **)&err, g_cond_err) != cudaSuccess) return false;
-  Args a{T, Ta, To, mat, patterns, reinterpret_cast<unsigned int *>(To), err, ncls, nx, ny, nz,
+  if (((int64_t)n_iter + 1) * b.nbx * b.nby + 1 >= COUNTER_LIMIT) return false;
+  int *err = wait_word(WAIT_CONDUCTION);
+  if (!err) return false;
+  Args a{T, Ta, To, mat, patterns, reinterpret_cast<unsigned int *>(To), err, 0, ncls, nx, ny, nz,
          b.nbx, b.nby, (int)pad, (int)cells, b.w * b.h, n_iter, P};
+  if (g_test_wait_error == 2) {
+    a.extra = 1;
+    g_test_wait_error = 0;
+  }
   const void *kernel = (const void *)be_resident_kernel<MatT, CLS>;
   if (!smem_opt_in(kernel, SMEM)) return false;
   if (cudaMemsetAsync(To, 0, 2 * sizeof(unsigned int), s) != cudaSuccess) return false;
@@ -1176,6 +1169,7 @@ int be_step(float *T, float *T_alt, float *T_old, const MatT *mat, int nx, int n
   if (st != BSP_OK) return st;
   if (!T_old) return BSP_ERR_NULL;
   if (n_iter < 0 || T == T_alt || T == T_old || T_alt == T_old) return BSP_ERR_ARG;
+  if (bsp::wait_status(bsp::WAIT_CONDUCTION) != BSP_OK) return BSP_ERR_TIMEOUT;
   const size_t bytes = sizeof(float) * (size_t)nx * ny * nz;
   const Params P{k, rho, cp, n_mat, dx, dt, h, tamb, mair};
   if (n_iter == 0)
@@ -1218,10 +1212,12 @@ bool launch_cls_tma(float *dst, const float *src, const float *told, float *snap
   if (SNAP) maps.o = maps.t;
   // the shared-memory opt-in is per device
   if (!smem_opt_in((const void *)be_cls_tma_kernel<SNAP>, TOTAL)) return false;
+  int *err = wait_word(WAIT_CONDUCTION);
+  if (!err) return false;
   const int bi = tma_bi(nx, ny, nz);
   dim3 grid((nz + 127) / 128, (ny + ROWS - 1) / ROWS, (nx + bi - 1) / bi);
   be_cls_tma_kernel<SNAP><<<grid, THREADS + 32, TOTAL, s>>>(dst, snap, maps, patterns, ncls,
-                                                            tiles, nx, ny, nz, bi, P);
+                                                            tiles, nx, ny, nz, bi, P, err);
   return cudaGetLastError() == cudaSuccess;
 }
 
@@ -1390,6 +1386,7 @@ extern "C" int bsp_conduction_be_cls(float *T, float *T_alt, float *T_old, const
   if (st != BSP_OK) return st;
   if (!T_old) return BSP_ERR_NULL;
   if (n_iter < 0 || T == T_alt || T == T_old || T_alt == T_old) return BSP_ERR_ARG;
+  if (bsp::wait_status(bsp::WAIT_CONDUCTION) != BSP_OK) return BSP_ERR_TIMEOUT;
   const size_t bytes = sizeof(float) * (size_t)nx * ny * nz;
   const Params P{k, rho, cp, n_mat, dx, dt, h_conv_air, T_amb, mat_air};
   if (n_iter == 0) return (int)cudaMemcpyAsync(T_old, T, bytes, cudaMemcpyDeviceToDevice, s);
@@ -1411,13 +1408,8 @@ extern "C" int bsp_conduction_be_cls(float *T, float *T_alt, float *T_old, const
 
 extern "C" int bsp_conduction_error(int *flag_host) {
   if (!flag_host) return BSP_ERR_NULL;
-  int v = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&v, bsp::cond::g_cond_err, sizeof(int));
-  if (e == cudaSuccess) {
-    const int zero = 0;
-    e = cudaMemcpyToSymbol(bsp::cond::g_cond_err, &zero, sizeof(int));
-  }
-  *flag_host = v;
+  const cudaError_t e = cudaDeviceSynchronize();
+  *flag_host = bsp::wait_status(bsp::WAIT_CONDUCTION) != BSP_OK;
   return (int)e;
 }
 

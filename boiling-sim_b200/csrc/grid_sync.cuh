@@ -79,6 +79,30 @@ __device__ __forceinline__ bool grid_barrier(GridCtl *ctl) {
   return s_ok != 0;
 }
 
+// The same on one word that only grows, zero at launch: every CTA adds one and waits for
+// `target` arrivals.  By thread 0 of a CTA, between two CTA barriers; false when a CTA gave up
+// (bounded as above): that CTA sets the word's top bit, which ends the others' waits at once
+// and every later one.  Arrivals have to stay below COUNTER_LIMIT.
+constexpr unsigned int COUNTER_LIMIT = 1u << 31;
+__device__ __forceinline__ bool counter_barrier(unsigned int *word, unsigned int target) {
+  cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(*word);
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  cnt.fetch_add(1u, cuda::memory_order_relaxed);  // released by the fence
+  unsigned int spins = 0, v;
+  unsigned long long t0 = 0;
+  while ((v = cnt.load(cuda::memory_order_acquire)) < target) {
+    if ((++spins & 255u) == 0) {
+      const unsigned long long now = gs_global_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > BAR_TIMEOUT_NS || spins > BAR_SPIN_LIMIT) {
+        cnt.fetch_or(COUNTER_LIMIT, cuda::memory_order_relaxed);
+        return false;
+      }
+    }
+  }
+  return v < COUNTER_LIMIT;
+}
+
 // Sum K doubles over the block (fixed order) and store them at
 // partials[k * stride + blockIdx.x].  sh must hold 32*K doubles.
 template <int K>

@@ -10,6 +10,7 @@
 
 #include "bsp_common.cuh"
 #include "profile.cuh"
+#include "waits.cuh"
 
 namespace bsp {
 
@@ -115,6 +116,7 @@ extern "C" int bsp_jacobi_solve(float *p, float *p_tmp, const float *div_u, floa
   if (nx <= 0 || ny <= 0 || nz <= 0 || n_iter <= 0) return BSP_OK;
   if (!p || !p_tmp || !div_u || !mask) return BSP_ERR_NULL;
   if (p == p_tmp || rhs_ws == p || rhs_ws == p_tmp) return BSP_ERR_ALIAS;
+  if (bsp::wait_status(bsp::WAIT_SWEEPS) != BSP_OK) return BSP_ERR_TIMEOUT;
   return bsp::jacobi_solve_impl(p, p_tmp, div_u, rhs_ws, mask, nx, ny, nz, dx, dt, rho, n_iter,
                                 tblock, stream, false, false, nullptr);
 }

@@ -12,6 +12,7 @@
 // are left for the caller to read.
 #include "bsp_common.cuh"
 #include "profile.cuh"
+#include "waits.cuh"
 
 namespace bsp {
 
@@ -391,6 +392,7 @@ static int projection_jacobi(float *p, float *p_tmp, float *div_u, float *ux, fl
   if (!p || !p_tmp || !div_u || !ux || !uy || !uz || !mask) return BSP_ERR_NULL;
   if (!dims_ok(nx + 1, ny, nz)) return BSP_ERR_SHAPE;
   if (p == p_tmp) return BSP_ERR_ALIAS;
+  if (wait_status(WAIT_SWEEPS) != BSP_OK) return BSP_ERR_TIMEOUT;
   const size_t bytes = sizeof(float) * (size_t)nx * ny * nz;
   cudaError_t e = cudaMemsetAsync(p, 0, bytes, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(p_tmp, 0, bytes, stream);

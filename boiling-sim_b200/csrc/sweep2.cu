@@ -22,6 +22,7 @@
 #include "bsp_common.cuh"
 #include "profile.cuh"
 #include "tma.cuh"
+#include "waits.cuh"
 
 namespace bsp {
 
@@ -214,19 +215,11 @@ __global__ void __launch_bounds__(sw2::THREADS, 2) sweep2_kernel(
   }
   if (producer)  // confirm (bounded) that nothing is still in flight
     for (int p = max(pbase, plast - NST + 1); p <= plast; ++p) wait(p);
-  if (!ok && threadIdx.x == 0) atomicExch(err, 1);
+  if (!ok && threadIdx.x == 0) wait_gave_up(err);
 }
 
-// Set by a sweep2 CTA whose bounded TMA wait gave up (the outputs of that
-// launch are then not valid); read back by bsp_sweep2_error.
-__device__ int g_sweep2_err;
 int num_sms();
 int sweep_bi_set(int64_t n);  // plane chunk set for grids of n cells, or 0 (stencil.cu)
-
-int *sweep2_error_word() {
-  int *err = nullptr;
-  return cudaGetSymbolAddress((void **)&err, g_sweep2_err) == cudaSuccess ? err : nullptr;
-}
 
 // Two sweeps p0 -> out (rhs already hoisted, p0 zero off fluid).  False when
 // the TMA path cannot run (nz % 16 != 0, alignment, no driver entry point).
@@ -240,7 +233,7 @@ bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *
         make_map(&maps.r, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, rhs, nx, ny, nz, FW, R1)))
     return false;
   if (!smem_opt_in((const void *)sweep2_kernel, TOTAL)) return false;
-  int *err = sweep2_error_word();
+  int *err = wait_word(WAIT_SWEEPS);  // marked by a CTA whose TMA wait gave up
   if (!err) return false;
   const int64_t cols = (int64_t)((nz + 127) / 128) * ((ny + ROWS - 1) / ROWS);
   int bi = 16;
@@ -253,16 +246,9 @@ bool launch_sweep2(float *out, const float *p, const float *rhs, const uint8_t *
 
 }  // namespace bsp
 
-// Device flag of a sweep2 launch whose TMA wait timed out: 1 if any did since
-// the last call (the flag is cleared); synchronises the device.
 extern "C" int bsp_sweep2_error(int *flag_host) {
   if (!flag_host) return BSP_ERR_NULL;
-  int v = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&v, bsp::g_sweep2_err, sizeof(int));
-  if (e == cudaSuccess) {
-    const int zero = 0;
-    e = cudaMemcpyToSymbol(bsp::g_sweep2_err, &zero, sizeof(int));
-  }
-  *flag_host = v;
+  const cudaError_t e = cudaDeviceSynchronize();
+  *flag_host = bsp::wait_status(bsp::WAIT_SWEEPS) != BSP_OK;
   return (int)e;
 }

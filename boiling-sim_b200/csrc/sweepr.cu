@@ -23,11 +23,12 @@
 #include "f32x2.cuh"
 #include "grid_sync.cuh"
 #include "profile.cuh"
+#include "waits.cuh"
 
 namespace bsp {
 
 int num_sms();
-int *sweep2_error_word();  // device flag of a sweep that gave up a bounded wait (sweep2.cu)
+extern int g_test_wait_error;  // BSP_TUNE_TEST_WAIT_ERROR (stencil.cu)
 
 namespace swr {
 
@@ -40,9 +41,10 @@ struct Args {
   const float *rhs;
   const uint8_t *mask;
   unsigned int *bar;  // zero at launch
-  int *err;
+  int *err;           // marked when the barrier gave up
   int nx, ny, nz;
   int bi, bj;
+  int extra;      // arrivals beyond the CTAs that a barrier waits for (0, or the error test's 1)
   int n, rounds;  // sweeps, rounds (round r: n / rounds sweeps, one more while r < n % rounds)
 };
 
@@ -113,31 +115,13 @@ __device__ __forceinline__ Quad off_fluid_one(const Quad &v, uint32_t f) {
   return quad(c);
 }
 
-// One grid barrier on a counter that only grows: every CTA adds one, and waits
-// for `target` arrivals (bounded; err is set on a timeout, and then read by the
-// CTAs that wait).
-__device__ __forceinline__ bool round_barrier(unsigned int *bar, unsigned int target, int *err) {
+// A grid barrier by the whole CTA; false after one that gave up, whose result is lost.
+__device__ __forceinline__ bool round_barrier(const Args &a, unsigned int target) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(*bar);
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    cnt.fetch_add(1u, cuda::memory_order_release);
-    int ok = 1;
-    unsigned int spins = 0;
-    unsigned long long t0 = 0;
-    while (cnt.load(cuda::memory_order_acquire) < target) {
-      if ((++spins & 1023u) == 0) {
-        const unsigned long long now = gs_global_ns();
-        if (t0 == 0) t0 = now;
-        if (now - t0 > BAR_TIMEOUT_NS || spins > BAR_SPIN_LIMIT) {
-          atomicExch(err, 1);
-          ok = 0;
-          break;
-        }
-      }
-    }
-    s_ok = ok;
+    s_ok = counter_barrier(a.bar, target);
+    if (!s_ok) wait_gave_up(a.err);
   }
   __syncthreads();
   return s_ok != 0;
@@ -409,7 +393,7 @@ __global__ void __launch_bounds__(THREADS, 1) resident_sweeps_kernel(const Args 
       }
     }
     if (last) return;
-    if (!round_barrier(a.bar, (unsigned int)(rd + 1) * gridDim.x, a.err)) return;
+    if (!round_barrier(a, (unsigned int)(rd + 1) * gridDim.x + a.extra)) return;
     if (work) {
       Quad hv[HQ];
 #pragma unroll
@@ -500,9 +484,15 @@ bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *ma
                   ((uintptr_t)mask & 3u) == 0;
   const Plan pl = make_plan(nx, ny, nz, num_sms(), al);
   if (!pl.grid) return false;
-  int *err = sweep2_error_word();
+  const int rounds = (n + pl.T - 1) / pl.T;
+  if ((int64_t)rounds * pl.grid + 1 >= COUNTER_LIMIT) return false;
+  int *err = wait_word(WAIT_SWEEPS);
   if (!err) return false;
-  Args a{p, p_tmp, rhs, mask, bar, err, nx, ny, nz, pl.bi, pl.bj, n, (n + pl.T - 1) / pl.T};
+  Args a{p, p_tmp, rhs, mask, bar, err, nx, ny, nz, pl.bi, pl.bj, 0, n, rounds};
+  if (g_test_wait_error == 1) {
+    a.extra = 1;
+    g_test_wait_error = 0;
+  }
   *e = cudaMemsetAsync(bar, 0, sizeof(unsigned int), s);
   if (*e != cudaSuccess) return true;
   ProfScope ps(PROF_SWEEP, s);

@@ -96,6 +96,10 @@ extern "C" {
                                      or 4 (48 registers a thread) */
 #define BSP_TUNE_GROUP_SOLVE 29   /* to-tolerance solves of small grids in one launch: 1 on (default),
                                      0 off (the same bits) */
+/* Tests only: the next projection whose sweeps run in one launch (1), or the next
+ * such conduction step (2), waits for a block too many and gives up after 2 s (the key
+ * clears itself). */
+#define BSP_TUNE_TEST_WAIT_ERROR 30
 
 /* ------------------------------------------------------------------ */
 /* 1. reference-compatible launchers                                   */
@@ -208,8 +212,14 @@ int bsp_jacobi_solve(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
 /* 1 in *flag_host if a temporally blocked sweep pass, or a projection whose
  * sweeps ran in one launch (bsp_projection_jacobi), gave up a bounded
  * device-side wait since the last call (its output is then invalid); clears
- * the flag.  Synchronises the device.  No reference counterpart. */
+ * the flag.  Synchronises the device (bsp_wait_status does not).  No reference counterpart. */
 int bsp_sweep2_error(int *flag_host);
+
+/* BSP_ERR_TIMEOUT if a call of the kind (0: Jacobi sweeps, 1: conduction) gave up a bounded
+ * device-side wait since that was last reported, else BSP_OK; clears it.  Does not synchronise: to
+ * be asked once the call's stream has been waited for.  The next call of the kind asks
+ * too, and returns BSP_ERR_TIMEOUT without doing anything if an earlier one gave up. */
+int bsp_wait_status(int kind);
 
 /* Set an autotuner parameter (BSP_TUNE_*) for subsequent launches in this
  * process.  Not thread-safe against concurrent launches. */
@@ -508,8 +518,10 @@ int bsp_conduction_sweep_cls(float *T_dst, const float *T_iter, const float *T_o
                              const uint8_t *tiles, int nx, int ny, int nz, const float *k,
                              const float *rho, const float *cp, int n_mat, float dx, float dt,
                              float h_conv_air, float T_amb, int mat_air, cudaStream_t stream);
-/* Read and clear the device flag that a TMA-fed conduction sweep sets when a
- * bounded wait gave up (its results are then not valid); synchronous. */
+/* 1 in *flag_host if a conduction call gave up a bounded device-side wait (TMA-fed sweeps,
+ * or the barrier of a step in one launch) since that was last reported: by this call or as
+ * the next step's BSP_ERR_TIMEOUT.  The temperatures are then not valid; the snapshot of a
+ * step in one launch (T_old) is.  Synchronises the device. */
 int bsp_conduction_error(int *flag_host);
 int bsp_conduction_be_cls(float *T, float *T_alt, float *T_old, const uint8_t *cls,
                           const uint32_t *patterns, int n_classes, const uint8_t *tiles, int nx,
