@@ -1149,8 +1149,8 @@ bool launch(float *T, float *Ta, float *To, const MatT *mat, const uint32_t *pat
   if (!smem_opt_in(kernel, SMEM)) return false;
   if (cudaMemsetAsync(To, 0, 2 * sizeof(unsigned int), s) != cudaSuccess) return false;
   void *args[] = {&a};
-  if (cudaLaunchCooperativeKernel(kernel, dim3(b.nbx * b.nby), dim3(THREADS), args, (size_t)bytes,
-                                  s) == cudaSuccess)
+  if (launch_coop(kernel, dim3(b.nbx * b.nby), dim3(THREADS), args, (size_t)bytes, s) ==
+      cudaSuccess)
     return true;
   (void)cudaGetLastError();
   return false;

@@ -27,6 +27,23 @@ struct GridCtl {
   int pad[3];
 };
 
+// Cooperative launch that the device may refuse: the whole grid does not fit beside what
+// the process may use (an MPS share, a green context).  The caller then takes a form that
+// needs no co-residency.
+extern bool g_test_refuse_coop;  // BSP_TUNE_TEST_REFUSE_COOP (stencil.cu)
+inline cudaError_t launch_coop(const void *fn, dim3 grid, dim3 block, void **args, size_t smem,
+                               cudaStream_t s) {
+  if (g_test_refuse_coop) return cudaErrorCooperativeLaunchTooLarge;
+  return cudaLaunchCooperativeKernel(fn, grid, block, args, smem, s);
+}
+inline bool coop_refused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported &&
+      e != cudaErrorLaunchOutOfResources)
+    return false;
+  (void)cudaGetLastError();
+  return true;
+}
+
 constexpr unsigned long long BAR_TIMEOUT_NS = 2000000000ull;  // 2 s
 constexpr unsigned int BAR_SPIN_LIMIT = 1u << 26;              // polls, a second guard
 

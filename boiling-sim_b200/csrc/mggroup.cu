@@ -1005,8 +1005,8 @@ __global__ void __launch_bounds__(THREADS) unit_list_kernel(uint32_t *__restrict
 template <class T>
 cudaError_t launch(const Params &P, int ctas, cudaStream_t s) {
   void *args[] = {const_cast<Params *>(&P)};
-  return cudaLaunchCooperativeKernel((const void *)group_solve_kernel<T>, dim3((unsigned)ctas),
-                                     dim3(THREADS), args, 0, s);
+  return launch_coop((const void *)group_solve_kernel<T>, dim3((unsigned)ctas), dim3(THREADS), args,
+                     0, s);
 }
 
 }  // namespace grp

@@ -514,10 +514,11 @@ extern "C" cudaError_t pressure_solve_pcg_launch(
     r.scale = a.scale;
     r.tol2 = a.tol2;
     e = launch_pcg_resident(r, plan, 0);
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpy(&h, ctl, sizeof(GridCtl), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return e;
-    if (h.err == 0 && h.status == PR_AGAIN) {
+    const bool refused = coop_refused(e);
+    if (e != cudaSuccess && !refused) return e;
+    if (!refused) e = cudaMemcpy(&h, ctl, sizeof(GridCtl), cudaMemcpyDeviceToHost);
+    if (!refused && e != cudaSuccess) return e;
+    if (!refused && h.err == 0 && h.status == PR_AGAIN) {
       e = cudaMemsetAsync(ctl, 0, sizeof(GridCtl), 0);
       if (e != cudaSuccess) return e;
     }

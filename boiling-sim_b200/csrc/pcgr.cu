@@ -398,8 +398,8 @@ cudaError_t launch_pcg_resident(PcgrArgs &a, const PcgrPlan &plan, cudaStream_t 
       pcg_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM);
   if (e != cudaSuccess) return e;
   void *args[] = {&a};
-  return cudaLaunchCooperativeKernel((const void *)pcg_resident_kernel, dim3(a.nbx * a.nby),
-                                     dim3(PR_THREADS), args, plan.bytes, s);
+  return launch_coop((const void *)pcg_resident_kernel, dim3(a.nbx * a.nby), dim3(PR_THREADS), args,
+                     plan.bytes, s);
 }
 
 }  // namespace bsp

@@ -1381,7 +1381,10 @@ static int group_info(const BspBatchItem &it, int storage, BspSolveInfo *info, c
 }
 
 // Solves count instances (all eligible, levels set up) in launches of at most
-// GROUP_MAX; infos as in bsp_solve_batch.
+// GROUP_MAX; infos as in bsp_solve_batch.  GROUP_REFUSED: the device did not take the launch,
+// and nothing has run (every launch asks for the same number of CTAs); the kernels' solve has
+// all it needs in the same setup.
+constexpr int GROUP_REFUSED = -1;
 template <class T>
 static int solve_group(int count, const BspBatchItem *items, const BspSolveParams *prm,
                        BspSolveInfo *infos, cudaStream_t s) {
@@ -1438,6 +1441,7 @@ static int solve_group(int count, const BspBatchItem *items, const BspSolveParam
       if (e != cudaSuccess) return (int)e;
     }
     const cudaError_t e = launch_group_solve<T>(P, s);
+    if (b == 0 && coop_refused(e)) return GROUP_REFUSED;
     if (e != cudaSuccess) return (int)e;
     q0 += P.count;
   }
@@ -1459,15 +1463,22 @@ int solve_impl(void *ws, const uint8_t *mask, const float *div, float *p_out, in
     const Level<T> &c = cx.lv[cx.lo.L - 1];
     if ((int64_t)c.nx * c.ny * c.nz > COARSEST_MAX) return BSP_ERR_SHAPE;
   }
+  bool ready = false;
+  auto setup = [&]() {
+    ready = ready || (prm->reuse_setup && setup_cached(ws, mask, nx, ny, nz, prm->storage));
+    if (ready) return cudaSuccess;
+    const cudaError_t e = setup_levels<T>(cx, s);
+    if (e == cudaSuccess) remember_setup(ws, mask, nx, ny, nz, prm->storage);
+    ready = e == cudaSuccess;
+    return e;
+  };
   if (group_eligible(nx, ny, nz)) {
-    if (!(prm->reuse_setup && setup_cached(ws, mask, nx, ny, nz, prm->storage))) {
-      const cudaError_t e = setup_levels<T>(cx, s);
-      if (e != cudaSuccess) return (int)e;
-      remember_setup(ws, mask, nx, ny, nz, prm->storage);
-    }
+    const cudaError_t e = setup();
+    if (e != cudaSuccess) return (int)e;
     const BspBatchItem item{p_out, div, mask, nx, ny, nz, dx, dt, rho, ws, cx.lo.total};
     BspSolveInfo own{};  // the host-driven solve returns its status even without info
-    return solve_group<T>(1, &item, prm, info ? info : &own, s);
+    const int st = solve_group<T>(1, &item, prm, info ? info : &own, s);
+    if (st != GROUP_REFUSED) return st;
   }
   SolverState h{};
   h.tol = prm->tol;
@@ -1494,11 +1505,8 @@ int solve_impl(void *ws, const uint8_t *mask, const float *div, float *p_out, in
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // v lives on this stack frame
     if (e != cudaSuccess) return (int)e;
   }
-  if (!(prm->reuse_setup && setup_cached(ws, mask, nx, ny, nz, prm->storage))) {
-    e = setup_levels<T>(cx, s);
-    if (e != cudaSuccess) return (int)e;
-    remember_setup(ws, mask, nx, ny, nz, prm->storage);
-  }
+  e = setup();
+  if (e != cudaSuccess) return (int)e;
   double *x = (double *)(cx.base + cx.lo.x);
   float *eb = (float *)(cx.base + cx.lo.e);
   const int nbr = row_blocks((int64_t)nx * ny);
@@ -1771,12 +1779,9 @@ static int finish_info(const Ctx<T> &cx, BspSolveInfo *info, cudaStream_t s) {
 template <class T>
 int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams *prm,
                       BspSolveInfo *infos, cudaStream_t s) {
-  std::vector<Ctx<T>> cxs;
+  std::vector<Ctx<T>> all;
   // instances for the group kernel, the others for the graph
   std::vector<int> small_at, large_at;
-  GraphKey key;
-  key.v.push_back((uintptr_t)count);
-  key_params(key, prm);
   for (int q = 0; q < count; ++q) {
     const BspBatchItem &it = items[q];
     Ctx<T> cx = make_ctx<T>(it.workspace, it.mask, it.nx, it.ny, it.nz, prm->storage);
@@ -1789,23 +1794,32 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
       if (e != cudaSuccess) return (int)e;
       remember_setup(it.workspace, it.mask, it.nx, it.ny, it.nz, prm->storage);
     }
-    if (group_eligible(it.nx, it.ny, it.nz)) {
-      small_at.push_back(q);
-      continue;
+    (group_eligible(it.nx, it.ny, it.nz) ? small_at : large_at).push_back(q);
+    all.push_back(cx);
+  }
+  std::vector<BspBatchItem> small;
+  for (int q : small_at) small.push_back(items[q]);
+  if (!small.empty()) {  // before the graph; their results are read after it
+    const int st = solve_group<T>((int)small.size(), small.data(), prm,
+                                  large_at.empty() ? infos : nullptr, s);
+    if (st == GROUP_REFUSED) {
+      small.clear();
+      small_at.clear();
+      large_at.clear();
+      for (int q = 0; q < count; ++q) large_at.push_back(q);
+    } else if (st != BSP_OK || large_at.empty()) {
+      return st;
     }
-    large_at.push_back(q);
+  }
+  GraphKey key;
+  key.v.push_back((uintptr_t)count);
+  key_params(key, prm);
+  for (int q : large_at) {
+    const BspBatchItem &it = items[q];
     for (uintptr_t x : {(uintptr_t)it.workspace, (uintptr_t)it.mask, (uintptr_t)it.div,
                         (uintptr_t)it.p, (uintptr_t)it.nx, (uintptr_t)it.ny, (uintptr_t)it.nz})
       key.v.push_back(x);
     key_floats(key, it.dx, it.dt, it.rho);
-    cxs.push_back(cx);
-  }
-  std::vector<BspBatchItem> small;
-  for (int q : small_at) small.push_back(items[q]);
-  if (large_at.empty()) return solve_group<T>(count, small.data(), prm, infos, s);
-  if (!small.empty()) {  // before the graph; their results are read after it
-    const int st = solve_group<T>((int)small.size(), small.data(), prm, nullptr, s);
-    if (st != BSP_OK) return st;
   }
   std::lock_guard<std::mutex> lk(g_graph_mu);
   cudaGraphExec_t exec = graph_lookup(key);
@@ -1816,7 +1830,7 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
     for (size_t q = 0; q < large_at.size() && e == cudaSuccess; ++q) {
       std::vector<cudaGraphNode_t> deps;
       const BspBatchItem &it = items[large_at[q]];
-      e = append_solve<T>(cxs[q], it.div, it.p, it.dx, it.dt, it.rho, prm, g, deps);
+      e = append_solve<T>(all[large_at[q]], it.div, it.p, it.dx, it.dt, it.rho, prm, g, deps);
     }
     prof_suspend(false);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
@@ -1831,7 +1845,7 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
   if (!infos) return BSP_OK;  // asynchronous: results land in p when the stream reaches them
   std::vector<int> states(count, BSP_OK);
   for (size_t q = 0; q < large_at.size(); ++q)
-    states[large_at[q]] = finish_info<T>(cxs[q], &infos[large_at[q]], s);
+    states[large_at[q]] = finish_info<T>(all[large_at[q]], &infos[large_at[q]], s);
   for (size_t q = 0; q < small.size(); ++q)
     states[small_at[q]] = group_info(small[q], prm->storage, &infos[small_at[q]], s);
   for (int st : states)

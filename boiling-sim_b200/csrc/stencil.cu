@@ -500,6 +500,8 @@ int g_sweep_prefetch = 2;
 // BSP_TUNE_TEST_WAIT_ERROR (tests only): the next one-launch sweeps (1) or conduction step (2)
 // wait at their first barrier for one arrival that never comes
 int g_test_wait_error = 0;
+// BSP_TUNE_TEST_REFUSE_COOP (tests only): the one-launch forms find their launch refused
+bool g_test_refuse_coop = false;
 // Cells up to which a sweep's fields (13 B a cell) count as resident in L2.
 constexpr int64_t L2_SWEEP_CELLS = 10LL << 20;
 // What bsp_autotune_jacobi has chosen (bsp_common.cuh), by the size of its grid: the three
@@ -1001,6 +1003,10 @@ extern "C" int bsp_set_tuning(int key, int value) {
     case BSP_TUNE_COARSE_TRACE:
       if (value < 0 || value > 1) return BSP_ERR_ARG;
       bsp::g_coarse_trace = value != 0;
+      return BSP_OK;
+    case BSP_TUNE_TEST_REFUSE_COOP:
+      if (value < 0 || value > 1) return BSP_ERR_ARG;
+      bsp::g_test_refuse_coop = value != 0;
       return BSP_OK;
     case BSP_TUNE_TEST_WAIT_ERROR:
       if (value < 0 || value > 2) return BSP_ERR_ARG;

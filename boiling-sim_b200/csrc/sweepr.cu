@@ -467,14 +467,14 @@ cudaError_t launch(const Args &a, const Plan &p, bool al, cudaStream_t s) {
                       : (const void *)resident_sweeps_kernel<T, Q, RR, false>;
   if (!smem_opt_in(fn, SMEM_MAX)) return cudaErrorNotSupported;
   void *args[] = {const_cast<Args *>(&a)};
-  return cudaLaunchCooperativeKernel(fn, dim3((unsigned)p.grid), dim3(THREADS), args, p.smem, s);
+  return launch_coop(fn, dim3((unsigned)p.grid), dim3(THREADS), args, p.smem, s);
 }
 
 }  // namespace swr
 
 // n sweeps from p = p_tmp = 0 with the result in p.  False when the grid is
-// too large to stay resident, or bar (4 bytes of device memory that the call
-// may use) is missing: nothing has been launched then.
+// too large to stay resident, bar (4 bytes of device memory that the call may use) is
+// missing, or the launch is refused: nothing runs then.
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
                      int nz, int n, unsigned int *bar, cudaStream_t s, cudaError_t *e) {
   using namespace swr;
@@ -497,7 +497,7 @@ bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *ma
   if (*e != cudaSuccess) return true;
   ProfScope ps(PROF_SWEEP, s);
 #define R(T_, Q_, RR_) \
-  if (pl.T == T_ && pl.Q == Q_) return (*e = launch<T_, Q_, RR_>(a, pl, al, s)), true
+  if (pl.T == T_ && pl.Q == Q_) return *e = launch<T_, Q_, RR_>(a, pl, al, s), !coop_refused(*e)
   R(1, 2, true);
   R(1, 4, true);
   R(1, 8, true);

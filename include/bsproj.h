@@ -100,6 +100,10 @@ extern "C" {
  * such conduction step (2), waits for a block too many and gives up after 2 s (the key
  * clears itself). */
 #define BSP_TUNE_TEST_WAIT_ERROR 30
+/* Tests only: 1 makes every cooperative launch of a one-launch form (solve, sweeps,
+ * conduction step, on-chip PCG) be refused, as where the device has fewer SMs for the process
+ * than it reports; the other forms then run.  0 (default). */
+#define BSP_TUNE_TEST_REFUSE_COOP 31
 
 /* ------------------------------------------------------------------ */
 /* 1. reference-compatible launchers                                   */
