@@ -21,7 +21,8 @@ enum ProfClass {
   PROF_PROJ = 9,       // divergence, gradient subtract, no-slip, rhs
   PROF_UNET = 10,      // learned warm start: network layers, input packing, head
   PROF_MG_MID = 11,    // levels 1-2 of the V-cycle on the column tile kernels (split mode)
-  PROF_NCLASS = 12
+  PROF_GROUP = 12,     // to-tolerance solve of small grids in one launch
+  PROF_NCLASS = 13
 };
 
 bool prof_enabled();

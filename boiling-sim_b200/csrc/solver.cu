@@ -926,11 +926,11 @@ Ctx<T> make_ctx(void *ws, const uint8_t *mask, int nx, int ny, int nz, int stora
 // and at GROUP_CELLS, the largest size that was measured (331x327x201: 36.4 ms per
 // kernel, 13.5 ms by a group; 384x384x120: 10.7 and 10.5 ms).  Host-driven, graph and
 // batched solves of a grid all take the same side, so that they agree bit for bit.  The
-// per-kernel path also serves what the group kernel has not: per-kernel tracing,
-// trilinear transfers, the barrier-error test.
+// per-kernel path also serves what the group kernel has not: trilinear transfers and the
+// barrier-error test.  (BSP_TUNE_GROUP_SOLVE = 0 for a record of its kernels.)
 constexpr int64_t GROUP_CELLS = 24LL << 20;
 bool group_eligible(int nx, int ny, int nz) {
-  if (!g_group_solve || g_l0_trilinear || g_test_barrier_error || prof_enabled()) return false;
+  if (!g_group_solve || g_l0_trilinear || g_test_barrier_error) return false;
   if ((int64_t)nx * ny * nz > GROUP_CELLS) return false;
   const int64_t n1 = (int64_t)((nx + 1) / 2) * ((ny + 1) / 2) * ((nz + 1) / 2);
   if ((nz + 1) / 2 % 4 == 0 && (nz + 1) / 2 >= 64 && n1 >= 131072) return false;
@@ -1440,7 +1440,11 @@ static int solve_group(int count, const BspBatchItem *items, const BspSolveParam
       const cudaError_t e = cudaMemsetAsync(in.base + lo.cctl, 0, 64, s);
       if (e != cudaSuccess) return (int)e;
     }
-    const cudaError_t e = launch_group_solve<T>(P, s);
+    cudaError_t e;
+    {
+      ProfScope ps(PROF_GROUP, s);
+      e = launch_group_solve<T>(P, s);
+    }
     if (b == 0 && coop_refused(e)) return GROUP_REFUSED;
     if (e != cudaSuccess) return (int)e;
     q0 += P.count;

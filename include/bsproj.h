@@ -238,11 +238,13 @@ int bsp_get_tuning(int key, int *value);
  * level, 3 search direction + A ps, 4 CG vector update, 5 FP64 residual,
  * 6 FP64 iterate update, 7 coarse multigrid levels, 8 control / setup
  * kernels, 9 divergence / gradient / no-slip / rhs, 10 learned warm start
- * (network layers on the tensor cores, input packing, head).
+ * (network layers on the tensor cores, input packing, head), 11 coarse levels on the tile
+ * kernels, 12 the solve of small grids in one launch (with BSP_TUNE_GROUP_SOLVE = 0 they
+ * are recorded as the kernels 1 .. 8 instead).
  * bsp_profile_read waits for the recorded launches, writes the summed
  * milliseconds and launch counts of classes 0..nclass-1 and clears the
  * record. */
-#define BSP_PROF_NCLASS 12
+#define BSP_PROF_NCLASS 13
 /* Tracing of the one-launch coarse V-cycle (with BSP_TUNE_COARSE_TRACE = 1):
  * host[0 .. n) receives CTA 0's %globaltimer (ns) at each phase boundary of
  * the last cycle launched (0 in unused slots, at most 48), and the record is
