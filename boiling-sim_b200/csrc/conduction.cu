@@ -45,6 +45,7 @@
 #include "waits.cuh"
 
 namespace bsp {
+extern bool g_one_launch;      // BSP_TUNE_ONE_LAUNCH (stencil.cu)
 extern int g_test_wait_error;  // BSP_TUNE_TEST_WAIT_ERROR (stencil.cu)
 int num_sms();
 
@@ -1129,7 +1130,7 @@ constexpr int MIN_ITER = 3;
 template <class MatT, bool CLS>
 bool launch(float *T, float *Ta, float *To, const MatT *mat, const uint32_t *patterns, int ncls,
             int nx, int ny, int nz, const Params &P, int n_iter, cudaStream_t s) {
-  if (n_iter < MIN_ITER || nz < 2 || (int64_t)nx * ny * nz > (int64_t)SLOTS * THREADS * num_sms())
+  if (!g_one_launch || n_iter < MIN_ITER || nz < 2 || (int64_t)nx * ny * nz > (int64_t)SLOTS * THREADS * num_sms())
     return false;
   const BlockSplit b = split_blocks(nx, ny, num_sms());
   const int64_t pad = (int64_t)(b.w + 2) * (b.h + 2) * (nz + 2);

@@ -456,6 +456,7 @@ static cudaError_t launch_pcg(PcgArgs<MaskT> &a, int max_blocks, cudaStream_t s)
 // four-cell form of the PCG phases where it applies, 0 the one-cell form (the same
 // per-cell operations)
 bool g_pcg_quad = true;
+extern bool g_one_launch;  // BSP_TUNE_ONE_LAUNCH (stencil.cu)
 
 // dot_workspace layout (>= 4096 bytes): [0,64) GridCtl, [64, 64 + 8*3*nb) partials
 constexpr int COMPAT_MAX_BLOCKS = (4096 - 64) / 24;
@@ -508,7 +509,7 @@ extern "C" cudaError_t pressure_solve_pcg_launch(
   GridCtl h{};
   h.status = PR_AGAIN;
   PcgrPlan plan;
-  if (g_pcg_quad && pcg_resident_fits(nx, ny, nz, std::min(num_sms(), COMPAT_MAX_BLOCKS), plan)) {
+  if (g_pcg_quad && g_one_launch && pcg_resident_fits(nx, ny, nz, std::min(num_sms(), COMPAT_MAX_BLOCKS), plan)) {
     PcgrArgs r{a.p, a.div, a.mask, a.z, a.partials, a.ctl, {}, nx, ny, nz, a.mf, a.ma, a.max_iter};
     for (int q = 0; q < 7; ++q) r.outs[q] = dst[q];
     r.scale = a.scale;

@@ -497,6 +497,11 @@ __global__ void __launch_bounds__(256, VEC == 4 ? 5 : 6)
 // BSP_TUNE_SWEEP_PREFETCH: the ZNF sweep's L2 prefetch distance in planes
 // (0 off, 2 default, 3).
 int g_sweep_prefetch = 2;
+// BSP_TUNE_SWEEP_POINT: the point kernel by its rule (launch_sweep_znf), or never where the march
+// can run.
+bool g_sweep_point = true;
+// BSP_TUNE_ONE_LAUNCH: sweeps, conduction steps and PCG of small grids on chip where they fit.
+bool g_one_launch = true;
 // BSP_TUNE_TEST_WAIT_ERROR (tests only): the next one-launch sweeps (1) or conduction step (2)
 // wait at their first barrier for one arrival that never comes
 int g_test_wait_error = 0;
@@ -700,7 +705,7 @@ cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const
                    (((uintptr_t)mask & 3u) == 0);
   const int64_t n = (int64_t)nx * ny * nz;
   const int set = sweep_bi_set(n);
-  if (nx <= 65535 && (ny + 7) / 8 <= 65535 && (!vec || (n <= L2_SWEEP_CELLS && set == 0))) {
+  if (nx <= 65535 && (ny + 7) / 8 <= 65535 && (!vec || (n <= L2_SWEEP_CELLS && set == 0 && g_sweep_point))) {
     auto fn = vec ? (fill ? launch_point<4, true> : launch_point<4, false>)
                   : (fill ? launch_point<1, true> : launch_point<1, false>);
     return fn(out, p, rhs, mask, nx, ny, nz, pdl, s);
@@ -1003,6 +1008,14 @@ extern "C" int bsp_set_tuning(int key, int value) {
     case BSP_TUNE_COARSE_TRACE:
       if (value < 0 || value > 1) return BSP_ERR_ARG;
       bsp::g_coarse_trace = value != 0;
+      return BSP_OK;
+    case BSP_TUNE_ONE_LAUNCH:
+      if (value < 0 || value > 1) return BSP_ERR_ARG;
+      bsp::g_one_launch = value != 0;
+      return BSP_OK;
+    case BSP_TUNE_SWEEP_POINT:
+      if (value < 0 || value > 1) return BSP_ERR_ARG;
+      bsp::g_sweep_point = value != 0;
       return BSP_OK;
     case BSP_TUNE_TEST_REFUSE_COOP:
       if (value < 0 || value > 1) return BSP_ERR_ARG;

@@ -28,6 +28,7 @@
 namespace bsp {
 
 int num_sms();
+extern bool g_one_launch;      // BSP_TUNE_ONE_LAUNCH (stencil.cu)
 extern int g_test_wait_error;  // BSP_TUNE_TEST_WAIT_ERROR (stencil.cu)
 
 namespace swr {
@@ -478,7 +479,7 @@ cudaError_t launch(const Args &a, const Plan &p, bool al, cudaStream_t s) {
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
                      int nz, int n, unsigned int *bar, cudaStream_t s, cudaError_t *e) {
   using namespace swr;
-  if (!bar || n < 2 || (int64_t)nx * ny * nz > (8LL << 20)) return false;
+  if (!g_one_launch || !bar || n < 2 || (int64_t)nx * ny * nz > (8LL << 20)) return false;
   const bool al = nz % 4 == 0 &&
                   (((uintptr_t)p | (uintptr_t)p_tmp | (uintptr_t)rhs) & 15u) == 0 &&
                   ((uintptr_t)mask & 3u) == 0;

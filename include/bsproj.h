@@ -104,6 +104,11 @@ extern "C" {
  * conduction step, on-chip PCG) be refused, as where the device has fewer SMs for the process
  * than it reports; the other forms then run.  0 (default). */
 #define BSP_TUNE_TEST_REFUSE_COOP 31
+#define BSP_TUNE_ONE_LAUNCH 32    /* Jacobi sweeps, conduction steps and reference-compatible PCG of
+                                     small grids on chip in one launch: 1 where they fit (default),
+                                     0 never (the same bits; PCG: but for its sums' order) */
+#define BSP_TUNE_SWEEP_POINT 33   /* single Jacobi sweeps of grids in L2 without a march: 1 (default),
+                                     0 the march wherever its alignment allows (the same bits) */
 
 /* ------------------------------------------------------------------ */
 /* 1. reference-compatible launchers                                   */
