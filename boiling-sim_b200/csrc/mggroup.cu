@@ -31,7 +31,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <vector>
 
 #include "bsp_common.cuh"
 #include "grid_sync.cuh"
@@ -1029,15 +1028,15 @@ void launch_group_units(uint32_t *list, uint8_t *flag, const uint8_t *mask, int 
   grp::unit_list_kernel<<<1, grp::THREADS, 0, s>>>(list, flag, n);
 }
 
-// Shares `sms` CTAs out over P's instances by their cells (at least one each) and
-// launches.  P.count <= min(GROUP_MAX, sms).
+// Shares the CTAs out over P's instances by their cells (at least one each) and
+// launches.  P.count <= min(GROUP_MAX, the device's SMs).
 template <class T>
-cudaError_t launch_group_solve(grp::Params &P, cudaStream_t s) {
-  const int sms = num_sms();
+cudaError_t launch_group_solve(grp::Params &P, int ctas, cudaStream_t s) {
+  const int sms = std::min(std::max(ctas, P.count), num_sms());
   double cells = 0.0;
   for (int q = 0; q < P.count; ++q) cells += (double)P.in[q].nx * P.in[q].ny * P.in[q].nz;
   int used = 0;
-  std::vector<double> want(P.count);
+  double want[grp::GROUP_MAX];
   for (int q = 0; q < P.count; ++q) {
     want[q] = (double)P.in[q].nx * P.in[q].ny * P.in[q].nz / cells * sms;
     P.in[q].ncta = std::max(1, (int)want[q]);
@@ -1064,8 +1063,8 @@ cudaError_t launch_group_solve(grp::Params &P, cudaStream_t s) {
   return grp::launch<T>(P, first, s);
 }
 
-template cudaError_t launch_group_solve<float>(grp::Params &, cudaStream_t);
-template cudaError_t launch_group_solve<__half>(grp::Params &, cudaStream_t);
-template cudaError_t launch_group_solve<__nv_bfloat16>(grp::Params &, cudaStream_t);
+template cudaError_t launch_group_solve<float>(grp::Params &, int, cudaStream_t);
+template cudaError_t launch_group_solve<__half>(grp::Params &, int, cudaStream_t);
+template cudaError_t launch_group_solve<__nv_bfloat16>(grp::Params &, int, cudaStream_t);
 
 }  // namespace bsp

@@ -63,7 +63,8 @@ void launch_group_codes(uint8_t *code, const uint8_t *mask, int nx, int ny, int 
 size_t group_units(int nx, int ny, int nz);
 void launch_group_units(uint32_t *list, uint8_t *flag, const uint8_t *mask, int nx, int ny, int nz,
                         cudaStream_t s);
+// On at most `ctas` CTAs (at least one an instance).
 template <class T>
-cudaError_t launch_group_solve(grp::Params &P, cudaStream_t s);
+cudaError_t launch_group_solve(grp::Params &P, int ctas, cudaStream_t s);
 
 }  // namespace bsp

@@ -29,6 +29,7 @@
 
 #include <cstring>
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -1360,6 +1361,32 @@ static void remember_setup(const void *ws, const void *mask, int nx, int ny, int
 }
 
 // ---- one-launch solve of small grids (mggroup.cu) ---------------------------------
+// A solve that is waited for alone takes every SM: it ends soonest.  Solves in flight
+// together (one that is only enqueued, or another thread's waiting for its own) would then run one
+// after another, so each takes a share, and whole-quad grids above SHARED_CELLS go by
+// the kernels, whose launches overlap (but for graph solves that are waited for, of which one
+// runs at a time there); the bits are the same.  Measured as projections a second with
+// 1 / 2 / 3 / 6 in flight (FP16): 56x56x40 kernels 508 / 930 / 1306 / 2236, all SMs 731 / 755 / 774 / 786,
+// a fifth 641 / 1257 / 1805 / 3134; 96x96x64 kernels 388 / 716 / 951 / 1377, all 510 / 563 / 591 / 607,
+// a third 454 / 872 / 1271 / 1387; 128x128x96 kernels 227 / 376 / 504 / 698, a third
+// 226 / 431 / 624 / 690; 144x144x96 kernels 220 / 372 / 503 / 709, a third 176 / 335 / 489 / 532.
+// Ragged rows gain by a third at every size (150x150x101: 152 / 241 / 304 / 373 by kernels,
+// 179 / 337 / 486 / 538).
+constexpr int64_t SHARED_CELLS = 1600000, FIFTH_CELLS = 200000;
+static std::atomic<int> g_waiting{0};  // calls that wait for their solve
+struct SolveShare {
+  const bool waits, shared;
+  explicit SolveShare(bool w) : waits(w), shared((w ? g_waiting.fetch_add(1) > 0 : true)) {}
+  ~SolveShare() {
+    if (waits) g_waiting.fetch_sub(1);
+  }
+  int ctas(int64_t cells) const {
+    return !shared ? num_sms() : std::max(1, num_sms() / (cells <= FIFTH_CELLS ? 5 : 3));
+  }
+  bool by_kernels(int nx, int ny, int nz, const uint8_t *mask) const {
+    return shared && (int64_t)nx * ny * nz > SHARED_CELLS && column_layout(nx, ny, nz, mask);
+  }
+};
 static_assert(grp::MAXL == MAX_LEVELS && grp::COARSEST == COARSEST_CELLS, "group constants");
 static_assert(4 * grp::PSTRIDE <= 3 * PARTIAL_STRIDE, "the group's sums fit the partials");
 static_assert(sizeof(grp::Result) <= sizeof(SolverState), "the result takes the state's place");
@@ -1387,7 +1414,7 @@ static int group_info(const BspBatchItem &it, int storage, BspSolveInfo *info, c
 constexpr int GROUP_REFUSED = -1;
 template <class T>
 static int solve_group(int count, const BspBatchItem *items, const BspSolveParams *prm,
-                       BspSolveInfo *infos, cudaStream_t s) {
+                       BspSolveInfo *infos, int ctas, cudaStream_t s) {
   const int most = std::min(grp::GROUP_MAX, num_sms());
   const int launches = (count + most - 1) / most;
   for (int b = 0, q0 = 0; b < launches; ++b) {
@@ -1443,7 +1470,7 @@ static int solve_group(int count, const BspBatchItem *items, const BspSolveParam
     cudaError_t e;
     {
       ProfScope ps(PROF_GROUP, s);
-      e = launch_group_solve<T>(P, s);
+      e = launch_group_solve<T>(P, ctas, s);
     }
     if (b == 0 && coop_refused(e)) return GROUP_REFUSED;
     if (e != cudaSuccess) return (int)e;
@@ -1476,12 +1503,13 @@ int solve_impl(void *ws, const uint8_t *mask, const float *div, float *p_out, in
     ready = e == cudaSuccess;
     return e;
   };
-  if (group_eligible(nx, ny, nz)) {
+  const SolveShare share(true);
+  if (group_eligible(nx, ny, nz) && !share.by_kernels(nx, ny, nz, mask)) {
     const cudaError_t e = setup();
     if (e != cudaSuccess) return (int)e;
     const BspBatchItem item{p_out, div, mask, nx, ny, nz, dx, dt, rho, ws, cx.lo.total};
     BspSolveInfo own{};  // the host-driven solve returns its status even without info
-    const int st = solve_group<T>(1, &item, prm, info ? info : &own, s);
+    const int st = solve_group<T>(1, &item, prm, info ? info : &own, share.ctas(cx.n), s);
     if (st != GROUP_REFUSED) return st;
   }
   SolverState h{};
@@ -1786,6 +1814,7 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
   std::vector<Ctx<T>> all;
   // instances for the group kernel, the others for the graph
   std::vector<int> small_at, large_at;
+  const SolveShare share(infos != nullptr);
   for (int q = 0; q < count; ++q) {
     const BspBatchItem &it = items[q];
     Ctx<T> cx = make_ctx<T>(it.workspace, it.mask, it.nx, it.ny, it.nz, prm->storage);
@@ -1798,14 +1827,17 @@ int solve_graph_batch(int count, const BspBatchItem *items, const BspSolveParams
       if (e != cudaSuccess) return (int)e;
       remember_setup(it.workspace, it.mask, it.nx, it.ny, it.nz, prm->storage);
     }
-    (group_eligible(it.nx, it.ny, it.nz) ? small_at : large_at).push_back(q);
+    const bool small = group_eligible(it.nx, it.ny, it.nz) &&
+                       !(count == 1 && !infos && share.by_kernels(it.nx, it.ny, it.nz, it.mask));
+    (small ? small_at : large_at).push_back(q);
     all.push_back(cx);
   }
   std::vector<BspBatchItem> small;
   for (int q : small_at) small.push_back(items[q]);
   if (!small.empty()) {  // before the graph; their results are read after it
     const int st = solve_group<T>((int)small.size(), small.data(), prm,
-                                  large_at.empty() ? infos : nullptr, s);
+                                  large_at.empty() ? infos : nullptr,
+                                  count == 1 ? share.ctas(all[0].n) : num_sms(), s);
     if (st == GROUP_REFUSED) {
       small.clear();
       small_at.clear();
