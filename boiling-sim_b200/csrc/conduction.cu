@@ -823,13 +823,18 @@ int pick_bi(int nx, int ny, int nz) {
   return bi;
 }
 
+// The column kernel takes these fields (old: T_old, or where the snapshot goes).
+template <class MatT>
+bool columns(const float *dst, const float *src, const float *old, const MatT *mat, int nz) {
+  return nz % 4 == 0 && al16(dst) && al16(src) && al16(old) &&
+         (sizeof(MatT) == 4 ? al16(mat) : (((uintptr_t)mat & 3u) == 0));
+}
+
 template <class MatT, bool SNAP>
 cudaError_t launch_sweep(float *dst, const float *src, const float *told, float *snap,
                          const MatT *mat, int nx, int ny, int nz, const Params &P,
                          cudaStream_t s) {
-  const bool col_ok = nz % 4 == 0 && al16(dst) && al16(src) && (SNAP ? al16(snap) : al16(told)) &&
-                      (sizeof(MatT) == 4 ? al16(mat) : (((uintptr_t)mat & 3u) == 0));
-  if (col_ok) {
+  if (columns<MatT>(dst, src, SNAP ? snap : told, mat, nz)) {
     const int bi = g_cond_bi > 0 ? g_cond_bi : pick_bi(nx, ny, nz);
     dim3 grid((nz / 4 + 31) / 32, (ny + 7) / 8, (nx + bi - 1) / bi);
     if (nz % 128 == 0)
@@ -895,16 +900,16 @@ struct Args {
   unsigned int *bar;  // arrivals, leavers
   int *err;           // marked when the barrier gave up
   int extra;          // as in sweepr.cu
+  uint32_t idmask;    // bits of a neighbour's material id that count
   int ncls, nx, ny, nz, nbx, nby, pad, cap, cols, n_iter;
   Params P;
 };
 
 // A face's code in a key of material ids: the neighbour's id, 15 on the domain edge
-// (no gamma).  Ids are masked as by the kernels that take such a grid's sweeps one by one.
+// (no gamma).  Ids are masked as by the kernel that would take the sweeps one by one.
 template <class MatT>
 __device__ __forceinline__ uint32_t id_key(const MatT *m, int c, int i, int j, int k, int nx,
-                                           int ny, int nz) {
-  const uint32_t mask = nz % 4 == 0 ? TCOLS - 1 : MAXM - 1;
+                                           int ny, int nz, uint32_t mask) {
   auto code = [&](bool in, int off) { return in ? mbyte(m, c + off) & mask : (uint32_t)OOB; };
   return code(i > 0, -ny * nz) | code(i + 1 < nx, ny * nz) << 4 | code(j > 0, -nz) << 8 |
          code(j + 1 < ny, nz) << 12 | code(k > 0, -1) << 16 | code(k + 1 < nz, 1) << 20 |
@@ -985,7 +990,7 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
       const int at = (li + 1) * di + (lj + 1) * dk + 1 + k, c = gp[col] + at;
       const float t = a.T[c];
       live = !is_air(c);
-      if (!CLS && live) key = id_key(mat, c, i0 + li, j0 + lj, k, nx, ny, nz);
+      if (!CLS && live) key = id_key(mat, c, i0 + li, j0 + lj, k, nx, ny, nz, a.idmask);
       P0[at] = live ? t : tamb;
       if (!live) P1[at] = tamb;
       if (c > 1) a.To[c] = t;
@@ -1140,7 +1145,8 @@ bool launch(float *T, float *Ta, float *To, const MatT *mat, const uint32_t *pat
   if (((int64_t)n_iter + 1) * b.nbx * b.nby + 1 >= COUNTER_LIMIT) return false;
   int *err = wait_word(WAIT_CONDUCTION);
   if (!err) return false;
-  Args a{T, Ta, To, mat, patterns, reinterpret_cast<unsigned int *>(To), err, 0, ncls, nx, ny, nz,
+  Args a{T, Ta, To, mat, patterns, reinterpret_cast<unsigned int *>(To), err, 0,
+         columns<MatT>(Ta, T, To, mat, nz) ? TCOLS - 1u : MAXM - 1u, ncls, nx, ny, nz,
          b.nbx, b.nby, (int)pad, (int)cells, b.w * b.h, n_iter, P};
   if (g_test_wait_error == 2) {
     a.extra = 1;
