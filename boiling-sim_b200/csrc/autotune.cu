@@ -27,13 +27,10 @@ extern bool g_coarse_fused_enabled;
 bool group_eligible(int nx, int ny, int nz);
 int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                       const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
-                      int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero,
-                      unsigned int *bar);
+                      int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero);
 }  // namespace bsp
 
 namespace {
-
-__device__ unsigned int g_tune_bar;  // barrier word of the one-launch sweeps while they are timed
 
 struct Timer {
   cudaEvent_t a = nullptr, b = nullptr;
@@ -70,9 +67,6 @@ extern "C" int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, f
   SweepTune &tuned = g_sweep_tuned[sweep_size(n)];
   const SweepTune saved = tuned;
   SweepTune choice = saved;
-  unsigned int *bar = nullptr;  // barrier word of the one-launch form
-  cudaError_t be = cudaGetSymbolAddress((void **)&bar, g_tune_bar);
-  if (be != cudaSuccess) return (int)be;
   Timer t;
   float best = 1e30f;
   *n_out = 0;
@@ -90,7 +84,7 @@ extern "C" int bsp_autotune_jacobi(float *p, float *p_tmp, const float *div_u, f
         cudaMemsetAsync(p_tmp, 0, bytes, s);
         cudaEventRecord(t.a, s);
         st = jacobi_solve_impl(p, p_tmp, div_u, rhs_ws, mask, nx, ny, nz, dx, dt, rho, sweeps,
-                               tb, s, true, true, bar);
+                               tb, s, true, true);
         cudaEventRecord(t.b, s);
       }
       if (st == BSP_OK) st = (int)cudaEventSynchronize(t.b);

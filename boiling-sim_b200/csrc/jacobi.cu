@@ -34,12 +34,11 @@ extern SweepTune g_sweep_tuned[3];
 int sweep_size(int64_t n);
 // sweepr.cu: all sweeps in one launch; false when the grid does not fit
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
-                     int nz, int n, unsigned int *bar, cudaStream_t s, cudaError_t *e);
+                     int nz, int n, cudaStream_t s, cudaError_t *e);
 
 // n_iter sweeps p <-> p_tmp, result in p.  tblock 0 (and no depth tuned for this size): the
 // whole solve in one launch with the pressure resident in shared memory where
-// that fits (p and p_tmp start at zero, the right-hand side hoisted, and bar, 4
-// bytes of device memory for a grid barrier, given), else one sweep per
+// that fits (p and p_tmp start at zero, the right-hand side hoisted), else one sweep per
 // pass.  tblock >= 2 (or the autotuner's choice): with the right-hand side
 // hoisted and the source zero off fluid, pairs of sweeps run as one temporally
 // blocked pass (sweep2.cu): fusing sweeps there doubles the instruction work
@@ -47,8 +46,7 @@ bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *ma
 // bit-identical to single sweeps.
 int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
                       const uint8_t *mask, int nx, int ny, int nz, float dx, float dt, float rho,
-                      int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero,
-                      unsigned int *bar) {
+                      int n_iter, int tblock, cudaStream_t stream, bool p_zero, bool tmp_zero) {
   if (n_iter <= 0) return BSP_OK;
   const int64_t n = (int64_t)nx * ny * nz;
   if (rhs_ws) {
@@ -59,7 +57,7 @@ int jacobi_solve_impl(float *p, float *p_tmp, const float *div_u, float *rhs_ws,
       tblock > 0 ? tblock : (g_sweep_tblock > 1 ? g_sweep_tblock : g_sweep_tuned[sweep_size(n)].tblock);
   if (depth == 0 && rhs_ws && p_zero && tmp_zero) {
     cudaError_t e = cudaSuccess;
-    if (sweeps_resident(p, p_tmp, rhs_ws, mask, nx, ny, nz, n_iter, bar, stream, &e)) return (int)e;
+    if (sweeps_resident(p, p_tmp, rhs_ws, mask, nx, ny, nz, n_iter, stream, &e)) return (int)e;
   }
   float *cur = p, *oth = p_tmp;
   bool cur_zero = p_zero, oth_zero = tmp_zero;  // +0 off fluid
@@ -118,5 +116,5 @@ extern "C" int bsp_jacobi_solve(float *p, float *p_tmp, const float *div_u, floa
   if (p == p_tmp || rhs_ws == p || rhs_ws == p_tmp) return BSP_ERR_ALIAS;
   if (bsp::wait_status(bsp::WAIT_SWEEPS) != BSP_OK) return BSP_ERR_TIMEOUT;
   return bsp::jacobi_solve_impl(p, p_tmp, div_u, rhs_ws, mask, nx, ny, nz, dx, dt, rho, n_iter,
-                                tblock, stream, false, false, nullptr);
+                                tblock, stream, false, false);
 }

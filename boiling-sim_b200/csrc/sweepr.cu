@@ -9,7 +9,9 @@
 // of T columns, in shared memory over all sweeps.  A round is T sweeps (each
 // valid one column less far into the halo), the store of the band of T columns
 // along the tile's edge to global memory, a grid barrier and the load of the
-// neighbours' bands.  Only the last round stores whole tiles.  Bands alternate
+// neighbours' bands.  The barrier's word is p_tmp's first element, which no neighbour's halo
+// reaches (make_plan) and no band is stored to: memory of this call alone.  Only the last
+// round stores whole tiles.  Bands alternate
 // between p and p_tmp, so a CTA that runs ahead never overwrites a band that a
 // neighbour still reads.  Every update is the reference's arithmetic in the
 // reference's order: the result is bit-identical to single sweeps.
@@ -41,7 +43,6 @@ struct Args {
   float *p, *p_tmp;
   const float *rhs;
   const uint8_t *mask;
-  unsigned int *bar;  // zero at launch
   int *err;           // marked when the barrier gave up
   int nx, ny, nz;
   int bi, bj;
@@ -121,7 +122,7 @@ __device__ __forceinline__ bool round_barrier(const Args &a, unsigned int target
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_ok = counter_barrier(a.bar, target);
+    s_ok = counter_barrier(reinterpret_cast<unsigned int *>(a.p_tmp), target);
     if (!s_ok) wait_gave_up(a.err);
   }
   __syncthreads();
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1) resident_sweeps_kernel(const Args 
           if (end && (last || (f >> 28) < 2u * T)) {
             int k;
             const int64_t g = gofs((idx[q] - wbase) >> 4, k);
-            store4<AL>(out, g, k, nz, cen[q]);
+            if (last || g != 0) store4<AL>(out, g, k, nz, cen[q]);  // 0: the barrier's word
           }
         }
         if (!end) __syncthreads();
@@ -434,11 +435,13 @@ Plan make_plan(int nx, int ny, int nz, int sms, bool al) {
   for (int bi = 1; bi <= nx; ++bi) {
     const int gi = (nx + bi - 1) / bi;
     if (gi > sms) continue;
-    const int bj = std::max(1, (ny + sms / gi - 1) / (sms / gi));
-    if (bi > 3 * bj || bj > 3 * bi) continue;
+    const int bj0 = std::max(1, (ny + sms / gi - 1) / (sms / gi));
     for (int T = 1; T <= 4; ++T) {
-      // bands reach one neighbour only
-      if (bi < T || bj < T) continue;
+      // bands reach one neighbour only, and the grid's first column none: a tile is wider
+      // than a halo, or as wide as the grid
+      const int bj = std::max(bj0, std::min(ny, T + 1));
+      if (bi < T || bj < T || (bi == T && gi > 1)) continue;
+      if (bi > 3 * bj || bj > 3 * bi) continue;
       const int64_t region = (int64_t)(bi + 2 * T - 2) * (bj + 2 * T - 2) * kq;
       const int q = (int)((region + 31 + THREADS - 1) / THREADS);
       const int Q = q <= 2 ? 2 : (q <= 4 ? 4 : (q <= 8 ? 8 : (q <= 16 ? 16 : 0)));
@@ -473,13 +476,13 @@ cudaError_t launch(const Args &a, const Plan &p, bool al, cudaStream_t s) {
 
 }  // namespace swr
 
-// n sweeps from p = p_tmp = 0 with the result in p.  False when the grid is
-// too large to stay resident, bar (4 bytes of device memory that the call may use) is
-// missing, or the launch is refused: nothing runs then.
+// n sweeps from p = p_tmp = 0 with the result in p (p_tmp's first element is then a
+// count).  False when the grid is too large to stay resident or the launch is refused:
+// nothing runs then.
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
-                     int nz, int n, unsigned int *bar, cudaStream_t s, cudaError_t *e) {
+                     int nz, int n, cudaStream_t s, cudaError_t *e) {
   using namespace swr;
-  if (!g_one_launch || !bar || n < 2 || (int64_t)nx * ny * nz > (8LL << 20)) return false;
+  if (!g_one_launch || n < 2 || (int64_t)nx * ny * nz > (8LL << 20)) return false;
   const bool al = nz % 4 == 0 &&
                   (((uintptr_t)p | (uintptr_t)p_tmp | (uintptr_t)rhs) & 15u) == 0 &&
                   ((uintptr_t)mask & 3u) == 0;
@@ -489,13 +492,11 @@ bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *ma
   if ((int64_t)rounds * pl.grid + 1 >= COUNTER_LIMIT) return false;
   int *err = wait_word(WAIT_SWEEPS);
   if (!err) return false;
-  Args a{p, p_tmp, rhs, mask, bar, err, nx, ny, nz, pl.bi, pl.bj, 0, n, rounds};
+  Args a{p, p_tmp, rhs, mask, err, nx, ny, nz, pl.bi, pl.bj, 0, n, rounds};
   if (g_test_wait_error == 1) {
     a.extra = 1;
     g_test_wait_error = 0;
   }
-  *e = cudaMemsetAsync(bar, 0, sizeof(unsigned int), s);
-  if (*e != cudaSuccess) return true;
   ProfScope ps(PROF_SWEEP, s);
 #define R(T_, Q_, RR_) \
   if (pl.T == T_ && pl.Q == Q_) return *e = launch<T_, Q_, RR_>(a, pl, al, s), !coop_refused(*e)
