@@ -383,8 +383,11 @@ __global__ void cls_assign_kernel(uint8_t *__restrict__ cls, uint32_t *__restric
 }
 
 // Per-CTA class table: tab[2c] = (1 + sum gamma, g-x, g+x, g-y), tab[2c+1] =
-// (g+y, g-z, g+z, 1 / (1 + sum gamma)).  gamma of a material pair as in gamma_entry; EDGE and
-// ids >= n_mat give 0.  Class 0 (air) gets den 1 and zero gammas.
+// (g+y, g-z, g+z, y), y 0 or (RCP) the reciprocal for div_by: a division a class and CTA, which
+// the kernels of one sweep a launch would pay for at every launch (2 % of a sweep at
+// 180x180x124).  gamma of a material pair as in gamma_entry; EDGE and ids >= n_mat give 0.
+// Class 0 (air) gets den 1 and zero gammas.
+template <bool RCP = false>
 __device__ __forceinline__ void build_class_table(float4 *tab, float *gt,
                                                   const uint32_t *__restrict__ patterns, int ncls,
                                                   const Params &P) {
@@ -406,8 +409,9 @@ __device__ __forceinline__ void build_class_table(float4 *tab, float *gt,
     }
     const float den = __fadd_rn(1.0f, diag);
     tab[2 * c] = make_float4(den, g[0], g[1], g[2]);
-    // for div_by (which divides where this is 0; below 1 only with a negative gamma)
-    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], den >= 1.0f ? rcp_of(den) : 0.0f);
+    // (div_by divides where y is 0; den is below 1 only with a negative gamma)
+    const float y = RCP && den >= 1.0f ? rcp_of(den) : 0.0f;
+    tab[2 * c + 1] = make_float4(g[3], g[4], g[5], y);
   }
   __syncthreads();
 }
@@ -944,7 +948,7 @@ __global__ void __launch_bounds__(THREADS, 1) be_resident_kernel(const __grid_co
   const uint32_t mair = (uint32_t)a.P.mair;
   auto is_air = [&](int c) { return CLS ? (mbyte(mat, c) & CLS_AIR) != 0 : mbyte(mat, c) == mair; };
   if (CLS)
-    build_class_table(tab, gt, a.patterns, a.ncls, a.P);
+    build_class_table<true>(tab, gt, a.patterns, a.ncls, a.P);
   else
     build_table16(gt, a.P);
   float t01[2] = {0.0f, 0.0f};
