@@ -37,6 +37,11 @@ namespace swr {
 
 constexpr int THREADS = 512;
 constexpr int HQ = 2;  // halo quads a thread loads at once
+// Sweeps from which one launch is taken: making the lists costs about five launches (a
+// projection of 2 / 5 / 10 / 16 sweeps, single and in one launch, us: 58x58x38 34 / 42 / 48 / 62
+// and 39 / 43 / 53 / 63; 110x110x68 52 / 71 / 88 / 115 and 61 / 73 / 90 / 111; 130x131x97 75 / 111 /
+// 152 / 211 and 82 / 102 / 134 / 171).
+constexpr int MIN_SWEEPS = 10;
 constexpr int SMEM_MAX = 232448 - 1024;  // dynamic; the rest is static
 
 struct Args {
@@ -482,7 +487,7 @@ cudaError_t launch(const Args &a, const Plan &p, bool al, cudaStream_t s) {
 bool sweeps_resident(float *p, float *p_tmp, const float *rhs, const uint8_t *mask, int nx, int ny,
                      int nz, int n, cudaStream_t s, cudaError_t *e) {
   using namespace swr;
-  if (!g_one_launch || n < 2 || (int64_t)nx * ny * nz > (8LL << 20)) return false;
+  if (!g_one_launch || n < MIN_SWEEPS || (int64_t)nx * ny * nz > (8LL << 20)) return false;
   const bool al = nz % 4 == 0 &&
                   (((uintptr_t)p | (uintptr_t)p_tmp | (uintptr_t)rhs) & 15u) == 0 &&
                   ((uintptr_t)mask & 3u) == 0;

@@ -279,8 +279,8 @@ int bsp_enforce_no_slip(float *ux, float *uy, float *uz, const uint8_t *mask, in
 /* Whole Jacobi projection (fluid.py:612-734): zero p and p_tmp, divergence,
  * n_iter sweeps, gradient subtract, diagnostic divergence.  max|div| after
  * the projection is written to *max_div_dev (device float).  No host sync.
- * With tblock 0, grids that fit the SMs' shared memory (up to about 2 M cells)
- * run their sweeps in one cooperative launch.  What p_tmp holds afterwards is
+ * With tblock 0 and ten sweeps or more, grids that fit the SMs' shared memory (up
+ * to about 2 M cells) run their sweeps in one cooperative launch.  What p_tmp holds afterwards is
  * unspecified. */
 int bsp_projection_jacobi(float *p, float *p_tmp, float *div_u, float *ux, float *uy,
                           float *uz, const uint8_t *mask, int nx, int ny, int nz, float dx,

@@ -61,7 +61,7 @@ def _tune(shape):
     return F.autotune_jacobi(grid, F.allocate_fluid_workspace(grid), DT, RHO, sweeps=20)
 
 
-@pytest.mark.parametrize("n_iter", [2, 9])
+@pytest.mark.parametrize("n_iter", [2, 9, 10, 19])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("tblock", [0, 1])
 def test_small_grids_run_in_one_launch(cuda, shape, n_iter, tblock):
@@ -69,7 +69,7 @@ def test_small_grids_run_in_one_launch(cuda, shape, n_iter, tblock):
     mat, ux, uy, uz = _scene(shape)
     want = O.projection_jacobi(ux, uy, uz, mat, DX, DT, RHO, n_iter)
     p, launches = _project(mat, ux, uy, uz, n_iter)
-    assert launches == 1
+    assert launches == (1 if n_iter >= 10 else n_iter)  # fewer are faster one by one
     assert np.array_equal(p.view(np.uint32), want["p"].view(np.uint32))
 
 
@@ -83,7 +83,7 @@ def test_default_can_be_set(cuda):
         call("bsp_set_tuning", TBLOCK, 3)
     with pytest.raises(BspError):
         call("bsp_get_tuning", 999, ctypes.byref(value))
-    assert _project(*_scene((16, 16, 16)), 9)[1] == 1
+    assert _project(*_scene((16, 16, 16)), 12)[1] == 1
 
 
 def test_autotuner_times_the_one_launch_form(cuda):
@@ -94,7 +94,7 @@ def test_autotuner_times_the_one_launch_form(cuda):
     assert (rows[0]["plane_chunk"], rows[0]["sweeps_per_pass"]) == (0, 0)
     assert launches == 2 + 5 * 2 * 20 + 6 * 2 * 10
     best = min(rows, key=lambda r: r["ms_per_sweep"])["sweeps_per_pass"]
-    assert _project(*_scene((58, 58, 48)), 9)[1] == {0: 1, 1: 9, 2: 5}[best]
+    assert _project(*_scene((58, 58, 48)), 12)[1] == {0: 1, 1: 12, 2: 6}[best]
 
 
 def test_tuning_a_large_grid_leaves_the_small_ones_alone(cuda):
@@ -102,7 +102,7 @@ def test_tuning_a_large_grid_leaves_the_small_ones_alone(cuda):
     grid in L2 gives the same bits."""
     _tune((256, 256, 192))
     mat, ux, uy, uz = _scene((58, 58, 38))
-    want = O.projection_jacobi(ux, uy, uz, mat, DX, DT, RHO, 9)
-    p, launches = _project(mat, ux, uy, uz, 9)
+    want = O.projection_jacobi(ux, uy, uz, mat, DX, DT, RHO, 12)
+    p, launches = _project(mat, ux, uy, uz, 12)
     assert launches == 1
     assert np.array_equal(p.view(np.uint32), want["p"].view(np.uint32))
