@@ -650,9 +650,12 @@ int sweep_bi_set(int64_t n) {
   return g_sweep_bi > 0 ? g_sweep_bi : g_sweep_tuned[sweep_size(n)].bi;
 }
 
-static inline int pick_bi(int nx, int ny, int nz) {
+// Plane chunk: the longest that still gives `per_sm` CTAs an SM.  Eight for the stencils, sixteen
+// for the ZNF march (256x256x192: 89 us a launcher sweep with eight, 95 with sixteen;
+// 384x384x256: 88 us a ZNF sweep with eight, 84 with sixteen).
+static inline int pick_bi(int nx, int ny, int nz, int per_sm) {
   const int64_t cols = (int64_t)((nz / 4 + 31) / 32) * ((ny + 7) / 8);
-  const int64_t target = (int64_t)num_sms() * 16;
+  const int64_t target = (int64_t)num_sms() * per_sm;
   int bi = 64;
   while (bi > 4 && cols * ((nx + bi - 1) / bi) < target) bi >>= 1;
   return bi;
@@ -667,7 +670,7 @@ cudaError_t launch_stencil(float *out, const float *p, const float *div, const M
                       (OP == OP_SPMV || aligned16(div)) &&
                       (sizeof(MaskT) == 4 ? aligned16(mask) : (((uintptr_t)mask & 3u) == 0));
   if (col_ok) {
-    const int set = sweep_bi_set((int64_t)nx * ny * nz), bi = set > 0 ? set : pick_bi(nx, ny, nz);
+    const int set = sweep_bi_set((int64_t)nx * ny * nz), bi = set > 0 ? set : pick_bi(nx, ny, nz, 8);
     dim3 grid((nz / 4 + 31) / 32, (ny + 7) / 8, (nx + bi - 1) / bi);
     if (nz % 128 == 0)
       stencil_col_kernel<OP, MaskT, true><<<grid, 256, 0, s>>>(out, p, div, mask, nx, ny, nz, bi,
@@ -713,7 +716,7 @@ cudaError_t launch_sweep_znf(float *out, const float *p, const float *rhs, const
   if (!vec)
     return launch_stencil<OP_JACOBI_RHS, uint8_t>(out, p, rhs, mask, nx, ny, nz, 0.f, 1.f, 0.f,
                                                   BSP_FLUID, BSP_AIR, s);
-  const int bi = set > 0 ? set : pick_bi(nx, ny, nz);
+  const int bi = set > 0 ? set : pick_bi(nx, ny, nz, 16);
   dim3 grid((nz / 4 + 31) / 32, (ny + 7) / 8, (nx + bi - 1) / bi);
   if (nz % 128 == 0)
     (g_sweep_prefetch == 3   ? sweep_znf_kernel<true, 3>
