@@ -186,17 +186,19 @@ __device__ __forceinline__ int64_t extend_from(const uint8_t *__restrict__ m, in
 }
 
 // QUAD: four cells a thread (rows of whole quads, aligned fields), copied as one where
-// all are fluid.
+// all are fluid, in CTAs of 32 quads x 8 j and g.planes planes.  Single cells in CTAs of
+// 64 k x 4 j and eight planes (200x200x130: 24 us, 32 in the quads' shape).
 template <bool QUAD>
 __global__ void __launch_bounds__(BK *BJ) extend_kernel(float *__restrict__ T_ext,
                                                         const float *__restrict__ T,
                                                         const uint8_t *__restrict__ m, Geo g) {
   constexpr int N = QUAD ? 4 : 1;
-  const int nz = g.nz, k = (blockIdx.x * BK + threadIdx.x) * N;
-  const int j = blockIdx.y * BJ + threadIdx.y;
+  const int nz = g.nz, k = (blockIdx.x * blockDim.x + threadIdx.x) * N;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (k >= nz || j >= g.ny) return;
-  for (int ii = 0; ii < g.planes; ++ii) {
-    const int i = blockIdx.z * g.planes + ii;
+  const int planes = QUAD ? g.planes : PL;
+  for (int ii = 0; ii < planes; ++ii) {
+    const int i = blockIdx.z * planes + ii;
     if (i >= g.nx) break;
     const int64_t c = ((int64_t)i * g.ny + j) * nz + k;
     if (QUAD) {
@@ -237,12 +239,13 @@ cudaError_t launch_extend(float *T_ext, const float *T, const uint8_t *m, const 
                           cudaStream_t s) {
   const bool quad = g.nz % 4 == 0 && (((uintptr_t)T_ext | (uintptr_t)T) & 15u) == 0 &&
                     ((uintptr_t)m & 3u) == 0;
-  const int nk = quad ? g.nz / 4 : g.nz;
-  const dim3 grid((nk + BK - 1) / BK, (g.ny + BJ - 1) / BJ, (g.nx + g.planes - 1) / g.planes);
+  const int nk = quad ? g.nz / 4 : g.nz, bk = quad ? BK : 64, bj = quad ? BJ : 4;
+  const int planes = quad ? g.planes : PL;
+  const dim3 grid((nk + bk - 1) / bk, (g.ny + bj - 1) / bj, (g.nx + planes - 1) / planes);
   if (quad)
-    extend_kernel<true><<<grid, dim3(BK, BJ), 0, s>>>(T_ext, T, m, g);
+    extend_kernel<true><<<grid, dim3(bk, bj), 0, s>>>(T_ext, T, m, g);
   else
-    extend_kernel<false><<<grid, dim3(BK, BJ), 0, s>>>(T_ext, T, m, g);
+    extend_kernel<false><<<grid, dim3(bk, bj), 0, s>>>(T_ext, T, m, g);
   return cudaGetLastError();
 }
 
@@ -391,9 +394,9 @@ cudaError_t launch_velocity(int axis, float *u_new, const float *ux, const float
 }
 
 bool dims_ok(int nx, int ny, int nz) {
-  // grid.z = nx + 1 planes and grid.y = ceil((ny + 1) / BJ) rows must fit the launch limits;
-  // the samplers use 32-bit element offsets
-  return nx + 1 <= 65535 && (ny + 1 + BJ - 1) / BJ <= 65535 &&
+  // grid.z = nx + 1 planes and grid.y = ceil((ny + 1) / 4) rows (4: the fewest of a CTA) must
+  // fit the launch limits; the samplers use 32-bit element offsets
+  return nx + 1 <= 65535 && (ny + 1 + 3) / 4 <= 65535 &&
          (int64_t)(nx + 1) * (ny + 1) * (nz + 1) < (1LL << 31);
 }
 
