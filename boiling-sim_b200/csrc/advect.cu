@@ -295,6 +295,131 @@ __global__ void __launch_bounds__(BK *BJ, 5) advect_u_kernel(float *__restrict__
   }
 }
 
+// ---- one field of a large grid ------------------------------------------------------
+// From FIELD_CELLS cells: coordinates only from the tables, and the axes formed per thread, in
+// CTAs of 64 k x 4 j marching eight planes.  One field's march reuses a line
+// less often than four do, and shared axes then cost more than they save (single calls, axes per
+// thread / shared, us: T at 384x384x256 362 / 421, 256x256x192 131 / 156, 192x192x128 55 / 65; uz at
+// 256x256x192 142 / 165; below the line T at 150x150x100 34 / 32, 110x110x68 24 / 18).
+constexpr int64_t FIELD_CELLS = 3 << 20;
+namespace wide {
+
+constexpr int BK = 64, BJ = 4, PL = 8;
+
+// World and scaled coordinates of a CTA's lattice points, computed once per
+// CTA: p = origin + (idx + s) dx and g = (p - origin) / dx per axis for its
+// plane i, its BJ rows and its BK columns (they depend on the index only).
+struct Coords {
+  float px[PL], gx[PL], py[BJ], gy[BJ], pz[BK], gz[BK];
+};
+
+__device__ __forceinline__ void coords(Coords &c, float sx, float sy, float sz, const Geo &g) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  if (ty == 0) {
+    const int k = blockIdx.x * BK + tx;
+    const float p = __fadd_rn(g.oz, __fmul_rn(__fadd_rn((float)k, sz), g.dx));
+    c.pz[tx] = p;
+    c.gz[tx] = __fdiv_rn(__fsub_rn(p, g.oz), g.dx);
+  } else if (ty == 1 && tx < BJ) {
+    const int j = blockIdx.y * BJ + tx;
+    const float p = __fadd_rn(g.oy, __fmul_rn(__fadd_rn((float)j, sy), g.dx));
+    c.py[tx] = p;
+    c.gy[tx] = __fdiv_rn(__fsub_rn(p, g.oy), g.dx);
+  } else if (ty == 2 && tx < PL) {
+    const int i = blockIdx.z * PL + tx;
+    const float p = __fadd_rn(g.ox, __fmul_rn(__fadd_rn((float)i, sx), g.dx));
+    c.px[tx] = p;
+    c.gx[tx] = __fdiv_rn(__fsub_rn(p, g.ox), g.dx);
+  }
+  __syncthreads();
+}
+
+// The velocity at the point (three samples at its scaled coordinates) and the
+// backtraced point's scaled coordinates.
+__device__ __forceinline__ void backtrace(float &bx, float &by, float &bz, const Coords &c,
+                                          int ii, const float *__restrict__ ux,
+                                          const float *__restrict__ uy,
+                                          const float *__restrict__ uz, const Geo &g) {
+  const float px = c.px[ii], gx = c.gx[ii];
+  const float py = c.py[threadIdx.y], gy = c.gy[threadIdx.y];
+  const float pz = c.pz[threadIdx.x], gz = c.gz[threadIdx.x];
+  const float u = tri(ux, g.nx + 1, g.ny, g.nz, gx, gy, gz, 0.0f, 0.5f, 0.5f);
+  const float v = tri(uy, g.nx, g.ny + 1, g.nz, gx, gy, gz, 0.5f, 0.0f, 0.5f);
+  const float w = tri(uz, g.nx, g.ny, g.nz + 1, gx, gy, gz, 0.5f, 0.5f, 0.0f);
+  const float qx = __fsub_rn(px, __fmul_rn(u, g.dt));
+  const float qy = __fsub_rn(py, __fmul_rn(v, g.dt));
+  const float qz = __fsub_rn(pz, __fmul_rn(w, g.dt));
+  bx = __fdiv_rn(__fsub_rn(qx, g.ox), g.dx);
+  by = __fdiv_rn(__fsub_rn(qy, g.oy), g.dx);
+  bz = __fdiv_rn(__fsub_rn(qz, g.oz), g.dx);
+}
+
+__global__ void __launch_bounds__(BK *BJ) advect_T_kernel(
+    float *__restrict__ T_new, const float *__restrict__ T_true, const float *__restrict__ T_ext,
+    const float *__restrict__ ux, const float *__restrict__ uy, const float *__restrict__ uz,
+    const uint8_t *__restrict__ m, Geo g) {
+  __shared__ Coords cs;
+  const int k = blockIdx.x * BK + threadIdx.x, j = blockIdx.y * BJ + threadIdx.y;
+  coords(cs, 0.5f, 0.5f, 0.5f, g);
+  if (k >= g.nz || j >= g.ny) return;
+  for (int ii = 0; ii < PL; ++ii) {
+    const int i = blockIdx.z * PL + ii;
+    if (i >= g.nx) break;
+    const int64_t c = ((int64_t)i * g.ny + j) * g.nz + k;
+    if (!fluid(m, c)) {
+      T_new[c] = __ldg(T_true + c);
+      continue;
+    }
+    float bx, by, bz;
+    backtrace(bx, by, bz, cs, ii, ux, uy, uz, g);
+    T_new[c] = tri(T_ext, g.nx, g.ny, g.nz, bx, by, bz, 0.5f, 0.5f, 0.5f);
+  }
+}
+
+template <int AX>
+__global__ void __launch_bounds__(BK *BJ) advect_u_kernel(float *__restrict__ u_new,
+                                                          const float *__restrict__ ux,
+                                                          const float *__restrict__ uy,
+                                                          const float *__restrict__ uz,
+                                                          const uint8_t *__restrict__ m, Geo g) {
+  __shared__ Coords cs;
+  const int fxn = g.nx + (AX == 0), fyn = g.ny + (AX == 1), fzn = g.nz + (AX == 2);
+  const int k = blockIdx.x * BK + threadIdx.x, j = blockIdx.y * BJ + threadIdx.y;
+  const float sx = AX == 0 ? 0.0f : 0.5f, sy = AX == 1 ? 0.0f : 0.5f, sz = AX == 2 ? 0.0f : 0.5f;
+  coords(cs, sx, sy, sz, g);
+  if (k >= fzn || j >= fyn) return;
+  const float *__restrict__ u = AX == 0 ? ux : (AX == 1 ? uy : uz);
+  const int64_t pl = (int64_t)g.ny * g.nz;
+  for (int ii = 0; ii < PL; ++ii) {
+    const int i = blockIdx.z * PL + ii;
+    if (i >= fxn) break;
+    const int64_t f = ((int64_t)i * fyn + j) * fzn + k;
+    const int a = AX == 0 ? i : (AX == 1 ? j : k);
+    const int na = AX == 0 ? fxn : (AX == 1 ? fyn : fzn);
+    if (a == 0 || a == na - 1) {
+      u_new[f] = 0.0f;
+      continue;
+    }
+    const int64_t c1 = i * pl + (int64_t)j * g.nz + k;
+    const int64_t c0 = AX == 0 ? c1 - pl : (AX == 1 ? c1 - g.nz : c1 - 1);
+    if (!fluid(m, c0) && !fluid(m, c1)) {
+      u_new[f] = __ldg(u + f);
+      continue;
+    }
+    float bx, by, bz;
+    backtrace(bx, by, bz, cs, ii, ux, uy, uz, g);
+    u_new[f] = tri(u, fxn, fyn, fzn, bx, by, bz, sx, sy, sz);
+  }
+}
+
+// CTAs: 64 k x 4 j, PL planes each
+inline dim3 grid_pl(int nx, int ny, int nz) {
+  return dim3((unsigned)((nz + BK - 1) / BK), (unsigned)((ny + BJ - 1) / BJ),
+              (unsigned)((nx + PL - 1) / PL));
+}
+
+}  // namespace wide
+
 // All four fields in one march over the cells (the faces before them; the thread of
 // the last cell also zeroes the face behind it): the twelve velocity samples and four
 // backtraced ones of a cell read the same few lines, which four kernels
@@ -380,6 +505,14 @@ inline dim3 grid_pl(int nx, int ny, int nz, int planes) {
 
 cudaError_t launch_velocity(int axis, float *u_new, const float *ux, const float *uy,
                             const float *uz, const uint8_t *m, const Geo &g, cudaStream_t s) {
+  if ((int64_t)g.nx * g.ny * g.nz >= FIELD_CELLS) {
+    auto fn = axis == 0   ? wide::advect_u_kernel<0>
+              : axis == 1 ? wide::advect_u_kernel<1>
+                          : wide::advect_u_kernel<2>;
+    fn<<<wide::grid_pl(g.nx + (axis == 0), g.ny + (axis == 1), g.nz + (axis == 2)),
+         dim3(wide::BK, wide::BJ), 0, s>>>(u_new, ux, uy, uz, m, g);
+    return cudaGetLastError();
+  }
   const dim3 blk(BK, BJ);
   if (axis == 0)
     advect_u_kernel<0>
@@ -425,8 +558,12 @@ extern "C" int bsp_advect_temperature(float *T_new, const float *T_true, const f
   if (!dims_ok(nx, ny, nz) || !(dx > 0.0f)) return BSP_ERR_SHAPE;
   const Geo g{nx, ny, nz, planes_of(nx, ny, nz), ox, oy, oz, dx, dt, bsp::rcp_of(dx),
               bsp::div_least(bsp::rcp_of(dx))};
-  advect_T_kernel<<<grid_pl(nx, ny, nz, g.planes), dim3(BK, BJ), 0, s>>>(T_new, T_true, T_ext, ux,
-                                                                         uy, uz, mask, g);
+  if ((int64_t)nx * ny * nz >= FIELD_CELLS)
+    wide::advect_T_kernel<<<wide::grid_pl(nx, ny, nz), dim3(wide::BK, wide::BJ), 0, s>>>(
+        T_new, T_true, T_ext, ux, uy, uz, mask, g);
+  else
+    advect_T_kernel<<<grid_pl(nx, ny, nz, g.planes), dim3(BK, BJ), 0, s>>>(T_new, T_true, T_ext,
+                                                                           ux, uy, uz, mask, g);
   return (int)cudaGetLastError();
 }
 
