@@ -173,79 +173,88 @@ __device__ __forceinline__ bool fluid(const uint8_t *__restrict__ m, int64_t c) 
   return (__ldg(m + c) & BSP_MFLUID) != 0;
 }
 
-// The cell that cell (i, j, k) takes its temperature from: itself if fluid, else the
-// first fluid neighbour in the order -x, +x, -y, +y, -z, +z (the six flags are loaded
-// together), else itself.
-__device__ __forceinline__ int64_t extend_from(const uint8_t *__restrict__ m, int64_t c, int i,
-                                               int j, int k, int nx, int ny, int nz) {
+// A cell takes its temperature from itself if fluid, else from the first fluid neighbour
+// in the order -x, +x, -y, +y, -z, +z (the six flags are loaded together), else itself.
+// Single cells, in CTAs of 64 k x 4 j marching eight planes (200x200x130: 24 us; 32 us in the
+// quads' shape).
+constexpr int XK = 64, XJ = 4, XP = 8;
+__global__ void __launch_bounds__(XK *XJ) extend_cells_kernel(float *__restrict__ T_ext,
+                                                              const float *__restrict__ T,
+                                                              const uint8_t *__restrict__ m, int nx,
+                                                              int ny, int nz) {
+  const int k = blockIdx.x * XK + threadIdx.x, j = blockIdx.y * XJ + threadIdx.y;
+  if (k >= nz || j >= ny) return;
   const int64_t pl = (int64_t)ny * nz;
-  const bool f0 = i > 0 && fluid(m, c - pl), f1 = i < nx - 1 && fluid(m, c + pl);
-  const bool f2 = j > 0 && fluid(m, c - nz), f3 = j < ny - 1 && fluid(m, c + nz);
-  const bool f4 = k > 0 && fluid(m, c - 1), f5 = k < nz - 1 && fluid(m, c + 1);
-  return f0 ? c - pl : f1 ? c + pl : f2 ? c - nz : f3 ? c + nz : f4 ? c - 1 : f5 ? c + 1 : c;
-}
-
-// QUAD: four cells a thread (rows of whole quads, aligned fields), copied as one where
-// all are fluid, in CTAs of 32 quads x 8 j and g.planes planes.  Single cells in CTAs of
-// 64 k x 4 j and eight planes (200x200x130: 24 us, 32 in the quads' shape).
-template <bool QUAD>
-__global__ void __launch_bounds__(BK *BJ) extend_kernel(float *__restrict__ T_ext,
-                                                        const float *__restrict__ T,
-                                                        const uint8_t *__restrict__ m, Geo g) {
-  constexpr int N = QUAD ? 4 : 1;
-  const int nz = g.nz, k = (blockIdx.x * blockDim.x + threadIdx.x) * N;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (k >= nz || j >= g.ny) return;
-  const int planes = QUAD ? g.planes : PL;
-  for (int ii = 0; ii < planes; ++ii) {
-    const int i = blockIdx.z * planes + ii;
-    if (i >= g.nx) break;
-    const int64_t c = ((int64_t)i * g.ny + j) * nz + k;
-    if (QUAD) {
-      const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(m + c));
-      float4 t = __ldg(reinterpret_cast<const float4 *>(T + c));
-      constexpr uint32_t F = BSP_MFLUID;
-      if ((w & F * 0x01010101u) != F * 0x01010101u) {
-        const int64_t pl = (int64_t)g.ny * nz;
-        auto word = [&](bool in, int64_t off) {
-          return in ? __ldg(reinterpret_cast<const uint32_t *>(m + c + off)) : 0u;
-        };
-        const uint32_t w0 = word(i > 0, -pl), w1 = word(i < g.nx - 1, pl);
-        const uint32_t w2 = word(j > 0, -nz), w3 = word(j < g.ny - 1, nz);
-        const uint32_t km = k > 0 ? __ldg(m + c - 1) : 0u;
-        const uint32_t kp = k + 4 < nz ? __ldg(m + c + 4) : 0u;
-        const uint32_t w4 = w << 8 | km, w5 = w >> 8 | kp << 24;
-        auto from = [&](int q, float own) {
-          const uint32_t f = F << (8 * q);
-          if (w & f) return own;
-          const int64_t off = w0 & f   ? -pl
-                              : w1 & f ? pl
-                              : w2 & f ? -(int64_t)nz
-                              : w3 & f ? nz
-                              : w4 & f ? -1
-                              : w5 & f ? 1
-                                       : 0;
-          return off ? __ldg(T + c + q + off) : own;
-        };
-        t = make_float4(from(0, t.x), from(1, t.y), from(2, t.z), from(3, t.w));
-      }
-      *reinterpret_cast<float4 *>(T_ext + c) = t;
-    } else {
-      T_ext[c] = __ldg(T + (fluid(m, c) ? c : extend_from(m, c, i, j, k, g.nx, g.ny, nz)));
+  for (int ii = 0; ii < XP; ++ii) {
+    const int i = blockIdx.z * XP + ii;
+    if (i >= nx) break;
+    const int64_t c = i * pl + (int64_t)j * nz + k;
+    int64_t s = c;
+    if (!fluid(m, c)) {
+      const bool f0 = i > 0 && fluid(m, c - pl), f1 = i < nx - 1 && fluid(m, c + pl);
+      const bool f2 = j > 0 && fluid(m, c - nz), f3 = j < ny - 1 && fluid(m, c + nz);
+      const bool f4 = k > 0 && fluid(m, c - 1), f5 = k < nz - 1 && fluid(m, c + 1);
+      s = f0 ? c - pl : f1 ? c + pl : f2 ? c - nz : f3 ? c + nz : f4 ? c - 1 : f5 ? c + 1 : c;
     }
+    T_ext[c] = __ldg(T + s);
   }
 }
+
+// Four cells a thread (rows of whole quads, aligned fields), copied as one where all are
+// fluid.
+__global__ void __launch_bounds__(BK *BJ) extend_quads_kernel(float *__restrict__ T_ext,
+                                                              const float *__restrict__ T,
+                                                              const uint8_t *__restrict__ m,
+                                                              Geo g) {
+  const int nz = g.nz, k = (blockIdx.x * BK + threadIdx.x) * 4;
+  const int j = blockIdx.y * BJ + threadIdx.y;
+  if (k >= nz || j >= g.ny) return;
+  for (int ii = 0; ii < g.planes; ++ii) {
+    const int i = blockIdx.z * g.planes + ii;
+    if (i >= g.nx) break;
+    const int64_t c = ((int64_t)i * g.ny + j) * nz + k;
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(m + c));
+    float4 t = __ldg(reinterpret_cast<const float4 *>(T + c));
+    constexpr uint32_t F = BSP_MFLUID;
+    if ((w & F * 0x01010101u) != F * 0x01010101u) {
+      const int64_t pl = (int64_t)g.ny * nz;
+      auto word = [&](bool in, int64_t off) {
+        return in ? __ldg(reinterpret_cast<const uint32_t *>(m + c + off)) : 0u;
+      };
+      const uint32_t w0 = word(i > 0, -pl), w1 = word(i < g.nx - 1, pl);
+      const uint32_t w2 = word(j > 0, -nz), w3 = word(j < g.ny - 1, nz);
+      const uint32_t km = k > 0 ? __ldg(m + c - 1) : 0u;
+      const uint32_t kp = k + 4 < nz ? __ldg(m + c + 4) : 0u;
+      const uint32_t w4 = w << 8 | km, w5 = w >> 8 | kp << 24;
+      auto from = [&](int q, float own) {
+        const uint32_t f = F << (8 * q);
+        if (w & f) return own;
+        const int64_t off = w0 & f   ? -pl
+                            : w1 & f ? pl
+                            : w2 & f ? -(int64_t)nz
+                            : w3 & f ? nz
+                            : w4 & f ? -1
+                            : w5 & f ? 1
+                                     : 0;
+        return off ? __ldg(T + c + q + off) : own;
+      };
+      t = make_float4(from(0, t.x), from(1, t.y), from(2, t.z), from(3, t.w));
+    }
+    *reinterpret_cast<float4 *>(T_ext + c) = t;
+  }
+}
+
 cudaError_t launch_extend(float *T_ext, const float *T, const uint8_t *m, const Geo &g,
                           cudaStream_t s) {
   const bool quad = g.nz % 4 == 0 && (((uintptr_t)T_ext | (uintptr_t)T) & 15u) == 0 &&
                     ((uintptr_t)m & 3u) == 0;
-  const int nk = quad ? g.nz / 4 : g.nz, bk = quad ? BK : 64, bj = quad ? BJ : 4;
-  const int planes = quad ? g.planes : PL;
-  const dim3 grid((nk + bk - 1) / bk, (g.ny + bj - 1) / bj, (g.nx + planes - 1) / planes);
   if (quad)
-    extend_kernel<true><<<grid, dim3(bk, bj), 0, s>>>(T_ext, T, m, g);
+    extend_quads_kernel<<<dim3((g.nz / 4 + BK - 1) / BK, (g.ny + BJ - 1) / BJ,
+                               (g.nx + g.planes - 1) / g.planes),
+                          dim3(BK, BJ), 0, s>>>(T_ext, T, m, g);
   else
-    extend_kernel<false><<<grid, dim3(bk, bj), 0, s>>>(T_ext, T, m, g);
+    extend_cells_kernel<<<dim3((g.nz + XK - 1) / XK, (g.ny + XJ - 1) / XJ, (g.nx + XP - 1) / XP),
+                          dim3(XK, XJ), 0, s>>>(T_ext, T, m, g.nx, g.ny, g.nz);
   return cudaGetLastError();
 }
 
