@@ -70,7 +70,8 @@ class TolSolver:
               graph: bool = False, wait: bool = True, want_x64: bool = True) -> SolveResult:
         """Solve A p = b for the divergence ``div``.  ``graph=True`` runs the
         whole solve as one device-driven CUDA graph (built on the first call
-        with this set of buffers, replayed afterwards).  ``wait=False`` (with
+        with this set of buffers, replayed afterwards), or a small grid's in
+        one launch.  ``wait=False`` (with
         ``graph``, after the first solve on these buffers) only enqueues the
         graph: p is written when the stream reaches it and the returned
         result carries no iteration counts (status 0, counts -1).
@@ -132,8 +133,9 @@ class TolSolver:
 
 
 class BatchSolver:
-    """Many independent pot scenes (uneven sizes) solved by one graph launch
-    (``bsp_solve_batch``).  Each instance owns its workspace; the masks are
+    """Many independent pot scenes (uneven sizes) solved together
+    (``bsp_solve_batch``: small grids in one cooperative launch, the others as branches
+    of one CUDA graph).  Each instance owns its workspace; the masks are
     fixed for the solver's lifetime."""
 
     def __init__(self, masks, storage: str = "fp32"):

@@ -47,7 +47,8 @@ constexpr int BK = 32, BJ = 8, PL = 8;  // CTA: 32 k x 8 j, marching up to 8 pla
 // Planes a CTA marches.  Large grids: 8, whose samples reuse the lines of the plane before
 // (384x384x256: 1464 us a step with 8 or more, 1483 us with 4); below 16 M cells
 // the CTAs in flight count for more (256x256x160: 499 us with 2, 533 us with 1; 128x128x96:
-// 94 us with 1, 139 us with 16; 56x56x40: 34 us with 1, 36 us with 2).
+// 94 us with 1, 139 us with 16; 56x56x40, when four copies brought the fields back: 34 us with 1,
+// 36 us with 2).
 inline int planes_of(int nx, int ny, int nz) {
   const int64_t n = (int64_t)nx * ny * nz;
   return n < (2 << 20) ? 1 : n < (16 << 20) ? 2 : PL;

@@ -10,8 +10,9 @@
 // 148 CTAs, less over few), ten of them an iteration; the SMs are shared out over the
 // instances by their cells, so a batch's instances run side by side.
 //
-// Measured, per-kernel path -> here: 110x110x68 FP16 2.00 -> 1.29 ms, 16 uneven pots
-// FP32 43.4 -> 8.6 ms, 200x200x130 FP16 (rows of no whole quads, where the per-kernel path
+// Measured, per-kernel path -> here: 110x110x68 FP16 2.00 -> 1.31 ms, 16 uneven pots
+// FP32 12.7 -> 9.2 ms with their setups kept (39.9 ms instead of 47.0 with them made),
+// 200x200x130 FP16 (rows of no whole quads, where the per-kernel path
 // has no tiles) 10.3 -> 4.4 ms, 331x327x201 FP32 36.4 -> 13.5 ms, 384x384x120 BF16 10.7 ->
 // 10.5 ms.  An iteration at 110x110x68 is 110 k cycles: 33 k on level 0, 40 k on the
 // coarse levels (latency of one round each), 25 k of barriers; in a batch

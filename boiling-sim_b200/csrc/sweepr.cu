@@ -2,18 +2,17 @@
 // shared memory: one cooperative launch runs all sweeps (jacobi.cu, from p = 0,
 // rho dx^2 div / dt hoisted into rhs).
 //
-// A sweep of a small grid costs a launch and a chain of load latencies, and on
-// every grid whose pressure fits the SMs' shared memory (about 5 M cells) the
-// instructions that form global addresses outnumber the arithmetic.  Here a
+// A sweep of a small grid costs a launch and a chain of load latencies, and the
+// instructions that form global addresses outnumber the arithmetic.  Taken for grids whose
+// windows fit the SMs (make_plan: up to 2.1 M cells in rows of whole quads, 4.5 M in others): a
 // CTA (one per SM) owns bi x bj columns of the grid and keeps them, with a halo
 // of T columns, in shared memory over all sweeps.  A round is T sweeps (each
 // valid one column less far into the halo), the store of the band of T columns
 // along the tile's edge to global memory, a grid barrier and the load of the
 // neighbours' bands.  The barrier's word is p_tmp's first element, which no neighbour's halo
 // reaches (make_plan) and no band is stored to: memory of this call alone.  Only the last
-// round stores whole tiles.  Bands alternate
-// between p and p_tmp, so a CTA that runs ahead never overwrites a band that a
-// neighbour still reads.  Every update is the reference's arithmetic in the
+// round stores whole tiles.  Bands alternate between p and p_tmp, so a CTA that runs ahead
+// never overwrites a band that a neighbour still reads.  Every update is the reference's arithmetic in the
 // reference's order: the result is bit-identical to single sweeps.
 //
 // A thread owns up to Q quads (four k cells) of the tile and its halo, keeps

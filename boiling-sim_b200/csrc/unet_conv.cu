@@ -9,9 +9,10 @@
 // 16-channel chunks ascending inside a tap -- because the ReLU gradient takes
 // its mask from the sign of the rounded output: another order flips an output
 // near zero once in a few million, and with it a term of the gradients.
-// tcgen05 kernels of the same tiling gave the same times at these channel
-// counts (32 -> 32 at 64x64x48: 31 us; an M = 128 instruction costs the same at
-// N = 32 as at N = 96) in another order.
+// The data gradient, the same kernel, has no mask taken from it and could be summed in
+// another order.  With both on tcgen05 (27 taps by moved descriptors; then the three di
+// stacked along N) a layer's training pass of 32 -> 32 channels at 64x64x48 took 169 and 125 us,
+// 154 us here; 16 -> 16 at 128x128x96 took 473 us with the first, 293 here.
 //
 // Forward.  A tile is 8 k x 16 j voxels; a CTA marches along i with the tile's
 // input window (10 x 18 rows of all input channels) of each plane staged once by

@@ -279,8 +279,9 @@ int bsp_enforce_no_slip(float *ux, float *uy, float *uz, const uint8_t *mask, in
 /* Whole Jacobi projection (fluid.py:612-734): zero p and p_tmp, divergence,
  * n_iter sweeps, gradient subtract, diagnostic divergence.  max|div| after
  * the projection is written to *max_div_dev (device float).  No host sync.
- * With tblock 0 and ten sweeps or more, grids that fit the SMs' shared memory (up
- * to about 2 M cells) run their sweeps in one cooperative launch.  What p_tmp holds afterwards is
+ * With tblock 0 and ten sweeps or more, grids that fit the SMs' shared memory (up to
+ * 2.1 M cells in rows of whole quads, 4.5 M in others) run their sweeps in one
+ * cooperative launch.  What p_tmp holds afterwards is
  * unspecified. */
 int bsp_projection_jacobi(float *p, float *p_tmp, float *div_u, float *ux, float *uy,
                           float *uz, const uint8_t *mask, int nx, int ny, int nz, float dx,
@@ -331,7 +332,14 @@ typedef struct BspSolveParams {
   int reuse_setup;  /* 1: the mask is unchanged since the last solve on this workspace,
                        reuse its multigrid setup (coarse masks, coarsest inverse) */
   int use_graph;    /* 1: run the whole solve as one CUDA graph (conditional WHILE
-                       nodes, no host synchronisation; built once per pointer set) */
+                       nodes, no host synchronisation; built once per pointer set).  A grid
+                       of up to 24 M cells whose coarse levels take no tile kernels (in
+                       rows of whole quads about 2 M cells) is solved in one cooperative
+                       launch either way: the V-cycle's tuning keys choose nothing there but
+                       the order of its sums (FINE_COLUMN, COARSE_FUSED).  Alone it takes
+                       every SM; enqueued (info NULL) or beside another waiting solve, a
+                       share of them, or from 1.6 M cells in rows of whole quads the kernels.
+                       The answer is the same bits in every case. */
 } BspSolveParams;
 
 /* One instance of a batched solve. */
@@ -388,9 +396,9 @@ int bsp_dot_noalloc(const float *x, const float *y, int64_t n, double *result_de
                     cudaStream_t stream);
 
 /* Solves `count` independent systems (uneven sizes allowed, one workspace
- * each) with one CUDA graph launch: every instance is an independent branch
- * of the graph running its own refinement and CG loops as conditional WHILE
- * nodes, so small instances overlap on the GPU.  The graph is built on the
+ * each).  Small and ragged grids (bsp_solve_tol) share one cooperative launch per 24
+ * instances, a group of CTAs each; the others are branches of one CUDA graph, each running
+ * its own refinement and CG loops as conditional WHILE nodes, built on the
  * first call for a given item set and replayed afterwards.  If infos is
  * non-NULL the call waits for the batch and fills one BspSolveInfo per item
  * (returning the first non-OK status); otherwise it returns after the
