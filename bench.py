@@ -607,7 +607,7 @@ def run_learned(args, dev, rank, world, dist):
 def run_batched(args, dev, rank, world, dist):
     """64 pot instances of uneven sizes (seeded draw, 48^3 .. 128x128x96), each
     with its own seeded velocity field, solved FP32-stored to FP64 rel-residual
-    1e-6 by one graph launch per batch; compared with 64 sequential host-driven
+    1e-6 in cooperative launches of up to 24; compared with 64 sequential host-driven
     solves of the same instances.  value = instances/s of the batched launch."""
     import torch
 
@@ -629,7 +629,7 @@ def run_batched(args, dev, rank, world, dist):
         ps.append(torch.zeros_like(d))
         cells += mat.size
     batch = BatchSolver(masks, args.storage)
-    infos = batch.solve(divs, ps, 0.002, DT, RHO, tol=TOL)  # builds the graph
+    infos = batch.solve(divs, ps, 0.002, DT, RHO, tol=TOL)  # builds the setups
     for _ in range(max(0, args.warmup - 1)):
         batch.solve(divs, ps, 0.002, DT, RHO, tol=TOL, wait=False)
     torch.cuda.synchronize()
@@ -664,8 +664,7 @@ def run_batched(args, dev, rank, world, dist):
             "data": "synthetic",
             "config": {"workload": f"64 pot scenes, sizes 48^3..128x128x96 (seed {SEED}), "
                                    f"{cells} cells in total, dx 2 mm", "storage": args.storage,
-                       "launch": "one CUDA graph per batch (conditional WHILE loops per "
-                                 "instance)"},
+                       "launch": "one cooperative launch per 24 instances (a group of CTAs each)"},
             "sequential_host_driven": {"value": round(64e3 / seq_ms, 2), "unit": "instances/s",
                                        "ms_per_64": round(seq_ms, 3)},
             "worst_rel_residual_fp64": worst,
@@ -1216,7 +1215,7 @@ def main():
     ap.add_argument("--config", default="projection",
                     choices=["projection", "batched", "learned"],
                     help="projection: the headline 384x384x256 projection; batched: 64 uneven "
-                         "pot scenes (48^3 .. 128x128x96) solved by one graph launch; learned: "
+                         "pot scenes (48^3 .. 128x128x96) solved in cooperative launches; learned: "
                          "the U-Net warm start on the 192x192x128 pots (walls 2/3/4)")
     args = ap.parse_args()
     world = int(os.environ.get("WORLD_SIZE", "1"))

@@ -25,9 +25,9 @@
 // fields is one such march (advect_all_kernel).  The loads' latency and the
 // instructions bound it, and warps in flight hide the former: forms that keep the
 // corners of the plane before in registers, fetch planes ahead into L2 or take 64 registers
-// were 3 to 18 % slower.  Measured, a kernel per field -> here: 384x384x256 1.94 -> 1.46 ms a
-// step with the copies back, 256x256x160 647 -> 499 us,
-// 128x128x96 158 -> 92 us, 56x56x40 80 -> 23 us.
+// were 3 to 18 % slower.  Measured, a kernel per field -> here, with the fields brought back:
+// 384x384x256 1.94 -> 1.47 ms a step, 256x256x160 657 -> 502 us, 128x128x96 158 -> 92 us,
+// 56x56x40 80 -> 24 us.
 #include <cuda_runtime.h>
 
 #include "../../include/bsproj.h"
@@ -478,8 +478,8 @@ __global__ void __launch_bounds__(BK *BJ, 5) advect_all_kernel(
 
 // The advected fields back into place where advect_all_kernel has changed them (a
 // pot's air and walls are two fifths of its cells): one launch for small grids, where four
-// copies take longer (56x56x40: 29 us a step, 36 us with the copies; 1.5 mm scene: 114
-// and 121 us); on large ones the copies' streams are the faster (200x193x130: 285 us
+// copies take longer (56x56x40: 29 us a step, 36 us with the copies, both before the extension
+// went by quads; 1.5 mm scene: 114 and 121 us); on large ones the copies' streams are the faster (200x193x130: 285 us
 // both; 256x256x160: 527 and 499 us).
 constexpr int64_t COPY_KERNEL_CELLS = 5 << 20;
 __global__ void __launch_bounds__(BK *BJ) copy_back_kernel(
