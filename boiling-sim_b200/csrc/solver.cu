@@ -1355,9 +1355,12 @@ static bool setup_cached(const void *ws, const void *mask, int nx, int ny, int n
 static void remember_setup(const void *ws, const void *mask, int nx, int ny, int nz,
                            int storage) {
   std::lock_guard<std::mutex> lk(g_setup_mu);
-  if (g_setups.size() >= SETUPS_MAX) g_setups.clear();
-  g_setups[ws] = SetupKey{mask, nx, ny, nz, storage, g_fine_bi, (int)g_l0_trilinear, g_fine_ctas,
-                           group_eligible(nx, ny, nz)};
+  try {
+    if (g_setups.size() >= SETUPS_MAX) g_setups.clear();
+    g_setups[ws] = SetupKey{mask, nx, ny, nz, storage, g_fine_bi, (int)g_l0_trilinear, g_fine_ctas,
+                            group_eligible(nx, ny, nz)};
+  } catch (...) {  // no memory for the record: the next solve sets up again
+  }
 }
 
 // ---- one-launch solve of small grids (mggroup.cu) ---------------------------------
